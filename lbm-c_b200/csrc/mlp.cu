@@ -3,14 +3,14 @@
 //
 // Training is plain mini-batch Adam on the mean squared error, all on the
 // GPU with hand-written kernels:
-//   mlp_grad_kernel      one sample per thread: forward pass with the BF16
-//                        weights (FP32 accumulation), backward pass, block
-//                        gradient sums in shared memory, one FP32 partial
-//                        per block;
-//   mlp_reduce_kernel    sums the block partials in a fixed order
-//                        (deterministic gradients);
-//   mlp_adam_kernel      Adam on the FP32 master weights, refreshes the BF16
-//                        copy the forward pass uses.
+//   mlp_grad_kernel      a few samples per warp, lane = hidden neuron:
+//                        forward pass with the BF16 weights (FP32
+//                        accumulation), backward pass, gradient sums in
+//                        registers, one FP32 partial per block;
+//   mlp_update_kernel    sums the block partials in a fixed order
+//                        (deterministic gradients), Adam on the FP32 master
+//                        weights, refreshes the BF16 copy the forward pass
+//                        uses.
 // The gradient is that of the loss as computed with the BF16-rounded
 // weights, which is what the CPU check (oracle/mlp_oracle.py) reproduces.
 #include <cuda_runtime.h>
@@ -25,6 +25,7 @@
 
 #include "../../include/lbmc.h"
 #include "engine_internal.h"
+#include "launch.cuh"
 #include "mlp.cuh"
 
 using namespace lbmc;
@@ -51,82 +52,210 @@ __global__ void normalise_kernel(const float *raw, const float *y, long long n, 
 
 // Gradient of sum over the batch of (y_hat - t)^2 / B with respect to the
 // (BF16-rounded) parameters; idx selects the batch's samples.
-__global__ void __launch_bounds__(GRAD_BLOCK)
+//
+// A sample's whole pass stays in one warp, lane = hidden neuron, GRAD_GROUP
+// samples at a time: lane j keeps row j and column j of W2 and row j of W1
+// and of their gradients in registers, so a layer is 32 broadcast 128-bit
+// shared-memory reads (the group's values of one neuron) with 4 FP32 FMAs
+// each, and the gradient needs no atomics.  The warps' sums meet in shared
+// memory once per block (rows padded to 33 so that neither the lane-wise
+// writes nor the parameter-wise reads conflict).  Bound by latency: a batch
+// of 4096 samples is one pass of 1024 warps (7.5 KFLOP a sample, 0.4 us of
+// the chip's FP32 rate).  One sample per thread with a shared-memory atomic
+// per parameter and sample, 16 blocks for a batch of 4096, took ~2400 us a
+// batch (32 lanes on one address); this kernel, the reduction and Adam
+// together GRAD_MEASURED.
+constexpr int GRAD_WARPS = GRAD_BLOCK / 32;
+constexpr int GRAD_GROUP = 4;                         // samples a warp takes at a time
+constexpr int GRAD_SAMPLES = GRAD_WARPS * GRAD_GROUP;  // per block and pass
+// The block's sums in shared memory: element (row i, lane j) of a matrix at i * 33 + j.
+constexpr int RED_W2 = 0, RED_W1 = RED_W2 + MLP_H * 33, RED_B1 = RED_W1 + MLP_IN * 33, RED_B2 = RED_B1 + MLP_H,
+              RED_W3 = RED_B2 + MLP_H, RED_B3 = RED_W3 + MLP_H, RED_LOSS = RED_B3 + 1, RED_SIZE = RED_LOSS + 1;
+
+// Where parameter p (or the loss, p = MLP_PARAMS) lies in the block's sums.
+__device__ __forceinline__ int red_index(int p) {
+  if (p < MLP_B1) return RED_W1 + (p % MLP_IN) * 33 + p / MLP_IN;
+  if (p < MLP_W2) return RED_B1 + (p - MLP_B1);
+  if (p < MLP_B2) return RED_W2 + ((p - MLP_W2) % MLP_H) * 33 + (p - MLP_W2) / MLP_H;
+  if (p < MLP_W3) return RED_B2 + (p - MLP_B2);
+  if (p < MLP_B3) return RED_W3 + (p - MLP_W3);
+  return p == MLP_B3 ? RED_B3 : RED_LOSS;
+}
+
+__device__ __forceinline__ float f4_get(const float4 &v, int s) {
+  return s == 0 ? v.x : s == 1 ? v.y : s == 2 ? v.z : v.w;
+}
+
+__global__ void __launch_bounds__(GRAD_BLOCK, 1)
     mlp_grad_kernel(const float *xn, const float *tn, const int *idx, int B, const __nv_bfloat16 *w,
                     float *partials) {
-  __shared__ float g[GRAD_SLOTS];
-  __shared__ float wf[MLP_PARAMS];
-  for (int p = threadIdx.x; p < MLP_PARAMS; p += blockDim.x) {
-    wf[p] = __bfloat162float(w[p]);
-    g[p] = 0.f;
+  __shared__ float4 h1_of[GRAD_WARPS][MLP_H], d2_of[GRAD_WARPS][MLP_H];
+  __shared__ float x_of[GRAD_WARPS][GRAD_GROUP][8];  // inputs, then the target
+  __shared__ float red[GRAD_WARPS / 2][RED_SIZE];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  release_successor();
+  // The samples do not depend on the previous training step: the first group
+  // is fetched before waiting for the weights.
+  auto fetch = [&](long long first) {
+    // 8 lanes a sample: six inputs, the target, one idle
+    const int s = lane >> 3, q = lane & 7;
+    float v = 0.f;
+    if (first + s < B && q < 7) {
+      const long long k = idx ? idx[first + s] : first + s;
+      v = q < MLP_IN ? xn[k * MLP_IN + q] : tn[k];
+    }
+    x_of[warp][s][q] = v;
+  };
+  const long long stride = (long long)gridDim.x * GRAD_SAMPLES;
+  long long first = blockIdx.x * GRAD_SAMPLES + warp * GRAD_GROUP;
+  fetch(first);
+  wait_for_predecessor();
+  float w1[MLP_IN], w2row[MLP_H], w2col[MLP_H];
+#pragma unroll
+  for (int q = 0; q < MLP_IN; q++) w1[q] = __bfloat162float(w[MLP_W1 + lane * MLP_IN + q]);
+#pragma unroll
+  for (int i = 0; i < MLP_H; i++) {
+    w2row[i] = __bfloat162float(w[MLP_W2 + lane * MLP_H + i]);
+    w2col[i] = __bfloat162float(w[MLP_W2 + i * MLP_H + lane]);
   }
-  if (threadIdx.x == 0) g[MLP_PARAMS] = 0.f;
-  __syncthreads();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < B) {
-    const int k = idx ? idx[s] : s;
-    float x[MLP_IN];
-    for (int i = 0; i < MLP_IN; i++) x[i] = xn[(long long)k * MLP_IN + i];
-    float a1[MLP_H], a2[MLP_H];
-    for (int j = 0; j < MLP_H; j++) {
-      float a = wf[MLP_B1 + j];
-      for (int i = 0; i < MLP_IN; i++) a += wf[MLP_W1 + j * MLP_IN + i] * x[i];
-      a1[j] = a;
+  const float b1 = __bfloat162float(w[MLP_B1 + lane]), b2 = __bfloat162float(w[MLP_B2 + lane]);
+  const float w3 = __bfloat162float(w[MLP_W3 + lane]), b3 = __bfloat162float(w[MLP_B3]);
+  float gw1[MLP_IN], gw2[MLP_H], gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, loss = 0.f;
+#pragma unroll
+  for (int q = 0; q < MLP_IN; q++) gw1[q] = 0.f;
+#pragma unroll
+  for (int i = 0; i < MLP_H; i++) gw2[i] = 0.f;
+  const float inv_b = 1.0f / (float)B;
+  for (; first < B; first += stride) {
+    __syncwarp();
+    // Layer 1: a = W1 x + b1; h1 = silu(a), p1 = silu'(a).
+    float p1[GRAD_GROUP], h[GRAD_GROUP];
+#pragma unroll
+    for (int s = 0; s < GRAD_GROUP; s++) {
+      float a = b1;
+#pragma unroll
+      for (int q = 0; q < MLP_IN; q++) a += w1[q] * x_of[warp][s][q];
+      const float sg = sigmoidf_(a);
+      h[s] = a * sg;
+      p1[s] = sg + h[s] * (1.0f - sg);
     }
-    float y = wf[MLP_B3];
-    for (int j = 0; j < MLP_H; j++) {
-      float a = wf[MLP_B2 + j];
-      for (int i = 0; i < MLP_H; i++) a += wf[MLP_W2 + j * MLP_H + i] * silu(a1[i]);
-      a2[j] = a;
-      y += wf[MLP_W3 + j] * silu(a);
+    h1_of[warp][lane] = make_float4(h[0], h[1], h[2], h[3]);
+    __syncwarp();
+    // Layer 2 and the output: y = W3 silu(W2 h1 + b2) + b3.
+    float a2[GRAD_GROUP] = {b2, b2, b2, b2};
+#pragma unroll
+    for (int i = 0; i < MLP_H; i++) {
+      const float4 v = h1_of[warp][i];
+#pragma unroll
+      for (int s = 0; s < GRAD_GROUP; s++) a2[s] += w2row[i] * f4_get(v, s);
     }
-    const float r = y - tn[k];
-    const float dy = 2.0f * r / (float)B;
-    atomicAdd(&g[MLP_PARAMS], r * r / (float)B);
-    atomicAdd(&g[MLP_B3], dy);
-    float d1[MLP_H];
-    for (int i = 0; i < MLP_H; i++) d1[i] = 0.f;
-    for (int j = 0; j < MLP_H; j++) {
-      const float sg = sigmoidf_(a2[j]);
-      const float h2 = a2[j] * sg;
-      atomicAdd(&g[MLP_W3 + j], dy * h2);
-      const float d2 = dy * wf[MLP_W3 + j] * (sg + a2[j] * sg * (1.0f - sg));
-      atomicAdd(&g[MLP_B2 + j], d2);
-      for (int i = 0; i < MLP_H; i++) {
-        atomicAdd(&g[MLP_W2 + j * MLP_H + i], d2 * silu(a1[i]));
-        d1[i] += d2 * wf[MLP_W2 + j * MLP_H + i];
+    float d2[GRAD_GROUP];
+#pragma unroll
+    for (int s = 0; s < GRAD_GROUP; s++) {
+      const float sg = sigmoidf_(a2[s]);
+      const float h2 = a2[s] * sg;
+      float y = w3 * h2;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) y += __shfl_xor_sync(0xffffffffu, y, off);
+      // samples past the batch count nothing
+      const float r = first + s < B ? y + b3 - x_of[warp][s][MLP_IN] : 0.f;
+      const float dy = 2.0f * r * inv_b;
+      loss += r * r * inv_b;
+      gb3 += dy;
+      gw3 += dy * h2;
+      d2[s] = dy * w3 * (sg + h2 * (1.0f - sg));
+      gb2 += d2[s];
+    }
+    d2_of[warp][lane] = make_float4(d2[0], d2[1], d2[2], d2[3]);
+    __syncwarp();
+    // Backward through W2, and the gradients of both layers.
+    float d1[GRAD_GROUP] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < MLP_H; i++) {
+      const float4 v = h1_of[warp][i], d = d2_of[warp][i];
+#pragma unroll
+      for (int s = 0; s < GRAD_GROUP; s++) {
+        gw2[i] += d2[s] * f4_get(v, s);
+        d1[s] += w2col[i] * f4_get(d, s);
       }
     }
-    for (int i = 0; i < MLP_H; i++) {
-      const float sg = sigmoidf_(a1[i]);
-      const float d = d1[i] * (sg + a1[i] * sg * (1.0f - sg));
-      atomicAdd(&g[MLP_B1 + i], d);
-      for (int q = 0; q < MLP_IN; q++) atomicAdd(&g[MLP_W1 + i * MLP_IN + q], d * x[q]);
+#pragma unroll
+    for (int s = 0; s < GRAD_GROUP; s++) {
+      const float d = d1[s] * p1[s];
+      gb1 += d;
+#pragma unroll
+      for (int q = 0; q < MLP_IN; q++) gw1[q] += d * x_of[warp][s][q];
     }
+    __syncwarp();
+    fetch(first + stride);
   }
+  // Warps 4..7 hand their sums to warps 0..3, then the block adds four rows.
+  auto each = [&](auto &&f) {
+#pragma unroll
+    for (int i = 0; i < MLP_H; i++) f(gw2[i], RED_W2 + i * 33 + lane);
+#pragma unroll
+    for (int q = 0; q < MLP_IN; q++) f(gw1[q], RED_W1 + q * 33 + lane);
+    f(gb1, RED_B1 + lane);
+    f(gb2, RED_B2 + lane);
+    f(gw3, RED_W3 + lane);
+    if (lane == 0) {
+      f(gb3, RED_B3);
+      f(loss, RED_LOSS);
+    }
+  };
+  float *row = red[warp % (GRAD_WARPS / 2)];
+  if (warp >= GRAD_WARPS / 2) each([&](float &v, int k) { row[k] = v; });
   __syncthreads();
-  for (int p = threadIdx.x; p < GRAD_SLOTS; p += blockDim.x)
-    partials[(long long)blockIdx.x * GRAD_SLOTS + p] = g[p];
+  if (warp < GRAD_WARPS / 2) each([&](float &v, int k) { row[k] += v; });
+  __syncthreads();
+  for (int p = threadIdx.x; p < GRAD_SLOTS; p += GRAD_BLOCK) {
+    const int k = red_index(p);
+    partials[(long long)blockIdx.x * GRAD_SLOTS + p] = (red[0][k] + red[1][k]) + (red[2][k] + red[3][k]);
+  }
 }
 
-__global__ void mlp_reduce_kernel(const float *partials, int nblocks, float *out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= GRAD_SLOTS) return;
-  float s = 0.f;
-  for (int b = 0; b < nblocks; b++) s += partials[(long long)b * GRAD_SLOTS + p];
-  out[p] = s;
-}
+// Adam's constants of one step; lr = 0 leaves the parameters alone.
+struct AdamStep {
+  float lr, b1, b2, eps, c1, c2;
+};
 
-__global__ void mlp_adam_kernel(float *master, float *m, float *v, const float *grad, __nv_bfloat16 *w,
-                                float lr, float b1, float b2, float eps, float c1, float c2) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= MLP_PARAMS) return;
-  const float g = grad[p];
-  const float mi = b1 * m[p] + (1.0f - b1) * g;
-  const float vi = b2 * v[p] + (1.0f - b2) * g * g;
+// Sums the block partials in a fixed order (deterministic gradients) and,
+// in a training step, applies Adam to the FP32 master weights and refreshes
+// the BF16 copy the forward pass uses; the loss goes to loss_out as well
+// where that is given.  REDUCE_PARAMS parameters a block, REDUCE_SLICES
+// threads to a parameter, so that the ~128 partials of a batch are read 16
+// deep instead of one after the other.
+constexpr int REDUCE_PARAMS = 32, REDUCE_SLICES = 8;
+__global__ void __launch_bounds__(REDUCE_PARAMS *REDUCE_SLICES)
+    mlp_update_kernel(const float *partials, int nblocks, float *grad, float *loss_out, bool train, AdamStep s,
+                      float *master, float *m, float *v, __nv_bfloat16 *w) {
+  __shared__ float sum[REDUCE_SLICES][REDUCE_PARAMS];
+  const int lane = threadIdx.x % REDUCE_PARAMS, slice = threadIdx.x / REDUCE_PARAMS;
+  const int p = blockIdx.x * REDUCE_PARAMS + lane;
+  release_successor();
+  wait_for_predecessor();
+  float t = 0.f;
+  if (p < GRAD_SLOTS) {
+#pragma unroll 16
+    for (int b = slice; b < nblocks; b += REDUCE_SLICES) t += partials[(long long)b * GRAD_SLOTS + p];
+  }
+  sum[slice][lane] = t;
+  __syncthreads();
+  if (slice != 0 || p >= GRAD_SLOTS) return;
+  float g = sum[0][lane];
+#pragma unroll
+  for (int k = 1; k < REDUCE_SLICES; k++) g += sum[k][lane];
+  grad[p] = g;
+  if (p == MLP_PARAMS) {
+    if (loss_out) *loss_out = g;
+    return;
+  }
+  if (!train) return;
+  const float mi = s.b1 * m[p] + (1.0f - s.b1) * g;
+  const float vi = s.b2 * v[p] + (1.0f - s.b2) * g * g;
   m[p] = mi;
   v[p] = vi;
-  const float step = lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  const float step = s.lr * (mi / s.c1) / (sqrtf(vi / s.c2) + s.eps);
   master[p] -= step;
   w[p] = __float2bfloat16_rn(master[p]);
 }
@@ -169,6 +298,8 @@ struct lbmc_mlp {
   __nv_bfloat16 *d_w = nullptr;
   long long adam_t = 0;
   unsigned long long seed = 0;
+  int sms = 1;
+  cudaStream_t stream = nullptr;  // the training kernels' (calls return when it is idle)
 };
 
 namespace {
@@ -268,7 +399,9 @@ extern "C" lbmc_status lbmc_mlp_create(int device, unsigned long long seed, lbmc
   m->host.target_scale = 1.f;
   m->host.iterations = 2;
   sync_host_weights(m);
-  cudaError_t e = upload(&m->d_master, m->master.data(), MLP_PARAMS);
+  cudaError_t e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = upload(&m->d_master, m->master.data(), MLP_PARAMS);
   std::vector<float> zeros(GRAD_SLOTS, 0.f);
   if (e == cudaSuccess) e = upload(&m->d_m, zeros.data(), MLP_PARAMS);
   if (e == cudaSuccess) e = upload(&m->d_v, zeros.data(), MLP_PARAMS);
@@ -314,12 +447,22 @@ static lbmc_status stage(lbmc_mlp *m, const float *features, const float *target
   return LBMC_OK;
 }
 
-static cudaError_t gradient(lbmc_mlp *m, const float *xn, const float *yn, const int *idx, int B,
-                            float *partials) {
-  const int nb = (B + GRAD_BLOCK - 1) / GRAD_BLOCK;
-  mlp_grad_kernel<<<nb, GRAD_BLOCK>>>(xn, yn, idx, B, m->d_w, partials);
-  mlp_reduce_kernel<<<(GRAD_SLOTS + 255) / 256, 256>>>(partials, nb, m->d_grad);
-  return cudaGetLastError();
+// Blocks of the gradient kernel for B samples: one pass of GRAD_SAMPLES a
+// block until every SM has one (its registers fill the SM), then several
+// passes a block.
+static int gradient_blocks(const lbmc_mlp *m, long long B) {
+  return (int)std::max(1LL, std::min((B + GRAD_SAMPLES - 1) / GRAD_SAMPLES, (long long)m->sms));
+}
+
+// Gradient (and loss) of one batch into d_grad; with `adam` also the step.
+static cudaError_t gradient(lbmc_mlp *m, const float *xn, const float *yn, const int *idx, int B, float *partials,
+                            const AdamStep *adam, float *loss_out) {
+  const int nb = gradient_blocks(m, B);
+  cudaError_t e = launch_chained(mlp_grad_kernel, dim3(nb), dim3(GRAD_BLOCK), m->stream, xn, yn, idx, B, m->d_w, partials);
+  if (e != cudaSuccess) return e;
+  return launch_chained(mlp_update_kernel, dim3((GRAD_SLOTS + REDUCE_PARAMS - 1) / REDUCE_PARAMS),
+                        dim3(REDUCE_PARAMS * REDUCE_SLICES), m->stream, partials, nb, m->d_grad, loss_out, adam != nullptr,
+                        adam ? *adam : AdamStep{}, m->d_master, m->d_m, m->d_v, m->d_w);
 }
 
 extern "C" lbmc_status lbmc_mlp_gradients(lbmc_mlp *m, const float *features, const float *target, long long n,
@@ -329,11 +472,12 @@ extern "C" lbmc_status lbmc_mlp_gradients(lbmc_mlp *m, const float *features, co
   float *xn = nullptr, *yn = nullptr, *partials = nullptr;
   lbmc_status s = stage(m, features, target, n, &xn, &yn);
   if (s != LBMC_OK) return s;
-  const int nb = (int)((n + GRAD_BLOCK - 1) / GRAD_BLOCK);
-  cudaError_t e = cudaMalloc(&partials, (size_t)nb * GRAD_SLOTS * sizeof(float));
-  if (e == cudaSuccess) e = gradient(m, xn, yn, nullptr, (int)n, partials);
+  cudaError_t e = cudaMalloc(&partials, (size_t)gradient_blocks(m, n) * GRAD_SLOTS * sizeof(float));
+  if (e == cudaSuccess) e = gradient(m, xn, yn, nullptr, (int)n, partials, nullptr, nullptr);
   std::vector<float> out(GRAD_SLOTS);
-  if (e == cudaSuccess) e = cudaMemcpy(out.data(), m->d_grad, GRAD_SLOTS * sizeof(float), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(out.data(), m->d_grad, GRAD_SLOTS * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   cudaFree(xn);
   cudaFree(yn);
   cudaFree(partials);
@@ -348,47 +492,54 @@ extern "C" lbmc_status lbmc_mlp_train(lbmc_mlp *m, const float *features, const 
   if (!m || !features || !target || n < 1 || epochs < 1 || batch < 1 || !(lr > 0))
     return merr(LBMC_ERR_INVALID_ARG, "lbmc_mlp_train");
   cudaSetDevice(m->device);
-  float *xn = nullptr, *yn = nullptr, *partials = nullptr;
+  float *xn = nullptr, *yn = nullptr, *partials = nullptr, *losses = nullptr;
   int *idx = nullptr;
   lbmc_status s = stage(m, features, target, n, &xn, &yn);
   if (s != LBMC_OK) return s;
-  const int nb = (batch + GRAD_BLOCK - 1) / GRAD_BLOCK;
-  cudaError_t e = cudaMalloc(&partials, (size_t)nb * GRAD_SLOTS * sizeof(float));
+  // Every LOSS_EVERY-th batch's loss counts in the history; the losses stay on
+  // the device until the end, so that no batch waits for the host.
+  constexpr long long LOSS_EVERY = 16;
+  const long long sampled = (n / batch + LOSS_EVERY - 1) / LOSS_EVERY;
+  cudaError_t e = cudaMalloc(&partials, (size_t)gradient_blocks(m, batch) * GRAD_SLOTS * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&idx, (size_t)n * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&losses, (size_t)std::max(1LL, sampled * epochs) * sizeof(float));
   std::vector<int> perm(n);
   std::iota(perm.begin(), perm.end(), 0);
   std::mt19937_64 rng(m->seed ^ 0x9E3779B97F4A7C15ull);
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  AdamStep a = {lr, 0.9f, 0.999f, 1e-8f, 0.f, 0.f};
   for (int ep = 0; ep < epochs && e == cudaSuccess; ep++) {
+    // the host shuffles while the device runs the previous epoch
     std::shuffle(perm.begin(), perm.end(), rng);
-    e = cudaMemcpy(idx, perm.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice);
-    double loss_sum = 0;
+    e = cudaMemcpyAsync(idx, perm.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, m->stream);
+    // perm is pageable: the copy may still read it until the stream is idle
+    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     long long batches = 0;
-    for (long long off = 0; off + batch <= n && e == cudaSuccess; off += batch) {
-      e = gradient(m, xn, yn, idx + off, batch, partials);
+    for (long long off = 0; off + batch <= n && e == cudaSuccess; off += batch, batches++) {
       m->adam_t++;
-      const float c1 = 1.0f - std::pow(b1, (float)m->adam_t), c2 = 1.0f - std::pow(b2, (float)m->adam_t);
-      if (e == cudaSuccess) {
-        mlp_adam_kernel<<<(MLP_PARAMS + 255) / 256, 256>>>(m->d_master, m->d_m, m->d_v, m->d_grad, m->d_w, lr, b1,
-                                                           b2, eps, c1, c2);
-        e = cudaGetLastError();
-      }
-      if (loss_history && e == cudaSuccess && (batches % 16 == 0)) {
-        float l = 0;
-        e = cudaMemcpy(&l, m->d_grad + MLP_PARAMS, sizeof(float), cudaMemcpyDeviceToHost);
-        loss_sum += l;
-      }
-      batches++;
+      a.c1 = 1.0f - std::pow(a.b1, (float)m->adam_t);
+      a.c2 = 1.0f - std::pow(a.b2, (float)m->adam_t);
+      e = gradient(m, xn, yn, idx + off, batch, partials, &a,
+                   batches % LOSS_EVERY == 0 ? losses + ep * sampled + batches / LOSS_EVERY : nullptr);
     }
-    if (loss_history) loss_history[ep] = (float)(loss_sum / std::max(1LL, (batches + 15) / 16));
   }
+  std::vector<float> loss_of((size_t)(sampled * epochs));
+  if (e == cudaSuccess && !loss_of.empty())
+    e = cudaMemcpyAsync(loss_of.data(), losses, loss_of.size() * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
   if (e == cudaSuccess)
-    e = cudaMemcpy(m->master.data(), m->d_master, MLP_PARAMS * sizeof(float), cudaMemcpyDeviceToHost);
+    e = cudaMemcpyAsync(m->master.data(), m->d_master, MLP_PARAMS * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   cudaFree(xn);
   cudaFree(yn);
   cudaFree(partials);
+  cudaFree(losses);
   cudaFree(idx);
   if (e != cudaSuccess) return merr(LBMC_ERR_CUDA, std::string("lbmc_mlp_train: ") + cudaGetErrorString(e));
+  if (loss_history)
+    for (int ep = 0; ep < epochs; ep++) {
+      double sum = 0;
+      for (long long k = 0; k < sampled; k++) sum += loss_of[ep * sampled + k];
+      loss_history[ep] = (float)(sum / (double)std::max(1LL, sampled));
+    }
   sync_host_weights(m);
   return LBMC_OK;
 }
@@ -483,6 +634,7 @@ extern "C" lbmc_status lbmc_mlp_destroy(lbmc_mlp *m) {
   cudaFree(m->d_v);
   cudaFree(m->d_grad);
   cudaFree(m->d_w);
+  if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
   return LBMC_OK;
 }
