@@ -12,6 +12,8 @@ namespace lbmc {
 // per SM.
 constexpr long long PIPE_STAGE_BUDGET = 32 * 1024;
 
+constexpr int B200_SMS = 148;
+
 template <class L, class S>
 struct Launchers {
   using C = typename Storage<S>::C;
@@ -54,6 +56,13 @@ struct Launchers {
     a.table = d.table_dev;
     a.closure = static_cast<const MlpStep *>(d.closure);
     a.mlp = d.closure_consts;
+    // The last blocks, as many as one wave of the chip holds, let the next
+    // step come up.
+    const long long per_row = grid_dim(d).x, rows = (long long)d.L[1] * d.L[2];
+    const long long wave = (long long)B200_SMS * (learned_closure(d.col)      ? direct_min_blocks<S, COL_BGK_MLP>()
+                                                  : d.col == COL_BGK_SMAG ? direct_min_blocks<S, COL_BGK_SMAG>()
+                                                                          : direct_min_blocks<S, COL_BGK>());
+    a.release_row = (int)(rows - (wave + per_row - 1) / per_row);
     a.sr_seed = sr_step_seed(t);
     return a;
   }
@@ -107,17 +116,13 @@ struct Launchers {
         return cudaSuccess;
       }
     }
-    if (!d.aa)
-      step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_SHIFT><<<grid_dim(d), block_dim(d), 0, st>>>(a);
-    else if (d.tiled && a.odd)
-      step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_ODD><<<grid_dim(d), block_dim(d), 0, st>>>(a);
-    else if (d.tiled)
-      step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_EVEN><<<grid_dim(d), block_dim(d), 0, st>>>(a);
-    else if (a.odd)
-      step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_ODD><<<grid_dim(d), block_dim(d), 0, st>>>(a);
-    else
-      step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_EVEN><<<grid_dim(d), block_dim(d), 0, st>>>(a);
-    return cudaSuccess;
+    auto run = [&](auto kern) { return launch_chained(kern, grid_dim(d), block_dim(d), st, a); };
+    if (!d.aa) return run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_SHIFT>);
+    if (d.tiled)
+      return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_ODD>)
+                   : run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_EVEN>);
+    return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_ODD>)
+                 : run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_EVEN>);
   }
 
   template <int COL, bool BLEND>

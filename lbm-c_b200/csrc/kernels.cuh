@@ -31,6 +31,7 @@
 #include <utility>
 
 #include "lattice.cuh"
+#include "launch.cuh"
 #include "mlp.cuh"
 
 namespace lbmc {
@@ -337,6 +338,7 @@ struct StepArgs {
   const uint16_t *table;        // 256 class-table entries (device memory)
   const MlpStep *closure;       // learned closure (COL_BGK_MLP, COL_BGK_MLP1): weights
   MlpConsts mlp;                // and its scalars
+  int release_row;              // direct kernel: block rows from here on release the next step
   unsigned sr_seed;             // stochastic-rounding seed of this step (sr_step_seed(t))
 };
 
@@ -1260,6 +1262,14 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   };
   double dv[DIAG_VALUES] = {0, 0, 0, 0, 0};
   bool nonfinite = false;
+  // The steps are chained (launch.cuh): the next step's blocks fill the SMs
+  // that this step's last blocks leave idle and read once it has completed
+  // (D2Q9 128x64: 4.10 -> 2.2 us a step, D3Q15 64^3: 8.2 -> 6.35, 256^3: the
+  // gap between steps is below 1%).  Only the last rows release it (an exited
+  // block counts as having done so): released from every block, the FP16
+  // 192^3 step took 115 instead of 103 us.  The class byte is read after the
+  // wait; before it, the learned closure's step was 5% slower.
+  if ((int)(blockIdx.y + gridDim.y * blockIdx.z) >= a.release_row) release_successor();
   if constexpr (!learned_closure(COL)) {
     if (!DIAG && !active) return;
     if (active) {
@@ -1270,6 +1280,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       const int n = x + a.L[0] * ((int)blockIdx.y + a.L[1] * (int)blockIdx.z);
       S *f = reinterpret_cast<S *>(a.f);
       Node<L, C> nd;
+      wait_for_predecessor();
       unroll<Q>([&](auto ic) { nd.g[decltype(ic)::value] = load_dev(read_at(f, st, ts, n, ic), inv_scale); });
       const int cls = a.cls[n];
       C out[Q];
@@ -1323,6 +1334,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       const int n = active ? x + a.L[0] * ((int)blockIdx.y + a.L[1] * (int)blockIdx.z) : 0;
       S *f = reinterpret_cast<S *>(a.f);
       Node<L, C> nd;
+      wait_for_predecessor();
       if (active) {
         init_sites(st, ts);
         unroll<Q>([&](auto ic) { nd.g[decltype(ic)::value] = load_dev(read_at(f, st, ts, n, ic), inv_scale); });
