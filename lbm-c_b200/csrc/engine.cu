@@ -33,6 +33,7 @@
 #include "kernels.cuh"
 #include "lattice.cuh"
 #include "mlp.cuh"
+#include "sweep.h"
 
 using namespace lbmc;
 
@@ -176,6 +177,9 @@ struct lbmc_handle {
   double *fetch_stage = nullptr;  // FP64 staging of uploads and lbmc_fetch (allocated on first use)
   long long fetch_stage_n = 0;
   std::vector<void *> allocations;
+  SweepPlan sweep;  // how steps are grouped; depth 1: one launch per step
+  cudaStream_t side_stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr, level_done[2][SweepPlan::MAX_DEPTH] = {};
 };
 
 // ------------------------------------------------------------ validation
@@ -531,6 +535,12 @@ static void release(lbmc_handle *h) {
   for (void *p : h->allocations) cudaFree(p);
   h->allocations.clear();
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
+  if (h->side_stream) cudaStreamDestroy(h->side_stream);
+  for (cudaEvent_t ev : {h->fork, h->join})
+    if (ev) cudaEventDestroy(ev);
+  for (auto &row : h->level_done)
+    for (cudaEvent_t ev : row)
+      if (ev) cudaEventDestroy(ev);
   delete h;
 }
 
@@ -565,6 +575,17 @@ static long long device_clock_khz(int device) {
     khz_of[device] = khz > 0 ? khz : 2000000;
   }
   return khz_of[device];
+}
+
+// Streams and events of a handle whose domain is swept (sweep.h).
+static cudaError_t make_sweep(lbmc_handle *h) {
+  cudaError_t e = cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking);
+  for (auto &row : h->level_done)
+    for (cudaEvent_t &ev : row)
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming);
+  return e;
 }
 
 extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom, lbmc_handle **out) {
@@ -757,6 +778,11 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
     TRYCUDA(cudaMemset(d.sf_buf, 0, (size_t)cs * q * d.n_sf), "clear sf");
   }
 
+  // Stress-free nodes need a pre-pass over the whole domain before each step,
+  // and the bulk-copy kernel walks all rows: both go step by step.
+  if (d.n_sf == 0 && !d.use_pipeline) h->sweep = plan_sweep(plane_count(d), n / plane_count(d) * q * ss, ss);
+  if (h->sweep.depth > 1) TRYCUDA(make_sweep(h), "sweep streams");
+
   // Initial populations (Init: model_builder.cu:227-248 for Init 0).
   if (cfg->init_type == LBMC_INIT_STATIC) {
     TRYCUDA(cudaMemset(d.f, 0, (size_t)d.pitch * q * ss), "clear populations");
@@ -835,18 +861,49 @@ __global__ void diag_finalize_kernel(const double *mid, double *out) {
   }
 }
 
+// `levels` steps in one sweep over the slabs; the side stream's work lies
+// between a fork from and a join with the handle's stream.
+static cudaError_t sweep(lbmc_handle *h, int levels) {
+  const SweepPlan &p = h->sweep;
+  const cudaStream_t st[2] = {h->stream, h->side_stream};
+  const int slabs = p.slabs(levels);
+  cudaError_t e = cudaEventRecord(h->fork, st[0]);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(st[1], h->fork, 0);
+  if (e != cudaSuccess) return e;
+  for (int k = 0; k < slabs && e == cudaSuccess; k++)
+    for (int s = 0; s < levels && e == cudaSuccess; s++) {
+      const int first = p.begin(k, s, levels), planes = p.end(k, s, levels) - first;
+      if (k > 0 && s > 0) e = cudaStreamWaitEvent(st[k & 1], h->level_done[(k - 1) & 1][s - 1], 0);
+      if (e == cudaSuccess)
+        e = h->ops->step(h->ds, h->step + s, false, false, first, planes, s < levels - 1, st[k & 1]);
+      if (e == cudaSuccess) e = cudaEventRecord(h->level_done[k & 1][s], st[k & 1]);
+    }
+  cudaError_t ej = cudaEventRecord(h->join, st[1]);
+  if (ej == cudaSuccess) ej = cudaStreamWaitEvent(st[0], h->join, 0);
+  if (e == cudaSuccess) e = ej;
+  if (e == cudaSuccess) h->step += levels;
+  return e;
+}
+
 extern "C" lbmc_status lbmc_iterate(lbmc_handle *h, int nsteps, unsigned flags) {
   if (!h) return fail(LBMC_ERR_INVALID_ARG, "lbmc_iterate: handle is NULL");
   if (nsteps < 0) return fail(LBMC_ERR_INVALID_ARG, "lbmc_iterate: nsteps = %d", nsteps);
   if (flags & ~(LBMC_STORE_MACROS | LBMC_REDUCE_DIAG | LBMC_SYNC))
     return fail(LBMC_ERR_INVALID_ARG, "lbmc_iterate: unknown flags 0x%x", flags);
   CK(cudaSetDevice(h->cfg.device), "cudaSetDevice");
-  for (int s = 0; s < nsteps; s++) {
+  // All steps but one that stores or reduces may run in sweeps.  (The learned
+  // closure's step is not bound by HBM.)
+  const int plain = nsteps - ((flags & (LBMC_STORE_MACROS | LBMC_REDUCE_DIAG)) ? 1 : 0);
+  const int depth = learned_closure(h->ds.col) ? 1 : h->sweep.depth;
+  int swept = 0;
+  for (int levels; depth > 1 && (levels = std::min(depth, plain - swept)) > 1; swept += levels)
+    CK(sweep(h, levels), "step kernel launch");
+  for (int s = swept; s < nsteps; s++) {
     const bool last = s == nsteps - 1;
     const bool store = last && (flags & LBMC_STORE_MACROS);
     const bool diag = last && (flags & LBMC_REDUCE_DIAG);
     if (diag) CK(cudaMemsetAsync(h->ds.flag, 0, sizeof(unsigned), h->stream), "clear flag");
-    CK(h->ops->step(h->ds, h->step, store, diag, h->stream), "step kernel launch");
+    CK(h->ops->step(h->ds, h->step, store, diag, 0, plane_count(h->ds), false, h->stream), "step kernel launch");
     h->step++;
     if (diag) {
       double *mid = h->ds.partials + DIAG_VALUES * h->nblocks;

@@ -51,11 +51,18 @@ struct DeviceState {
   lbmc::MlpConsts closure_consts;  // its scalars, passed with each launch
 };
 
+// Planes along the slowest axis (z in 3-D, y in 2-D).
+inline int plane_count(const DeviceState &d) { return d.L[d.dim - 1]; }
+
 struct LatticeStorageOps {
   int csize;  // bytes of the compute type
   int ssize;  // bytes of the storage type
-  // One time step at step counter t (shift t mod L).
-  cudaError_t (*step)(const DeviceState &, long long t, bool store, bool diag, cudaStream_t);
+  // One time step at step counter t (shift t mod L) of `planes` planes (z in
+  // 3-D, y in 2-D) from plane `first` on, wrapping past the last one; the
+  // whole domain with planes = plane_count().  keep: the next step follows
+  // while these planes are in L2.
+  cudaError_t (*step)(const DeviceState &, long long t, bool store, bool diag, int first, int planes, bool keep,
+                      cudaStream_t);
   // out[x] = f_i(x) in natural layout (FP64) at step counter t.
   cudaError_t (*fetch_population)(const DeviceState &, long long t, int i, double *out,
                                    cudaStream_t);

@@ -18,7 +18,7 @@ template <class L, class S>
 struct Launchers {
   using C = typename Storage<S>::C;
 
-  static StepArgs<C> make_args(const DeviceState &d, long long t, bool store) {
+  static StepArgs<C> make_args(const DeviceState &d, long long t, bool store, int first, int planes, bool keep) {
     StepArgs<C> a;
     a.f = d.f;
     a.pitch = d.pitch;
@@ -58,11 +58,13 @@ struct Launchers {
     a.mlp = d.closure_consts;
     // The last blocks, as many as one wave of the chip holds, let the next
     // step come up.
-    const long long per_row = grid_dim(d).x, rows = (long long)d.L[1] * d.L[2];
+    const long long per_row = grid_dim(d, planes).x, rows = (long long)planes * (d.dim == 3 ? d.L[1] : 1);
     const long long wave = (long long)B200_SMS * (learned_closure(d.col)      ? direct_min_blocks<S, COL_BGK_MLP>()
                                                   : d.col == COL_BGK_SMAG ? direct_min_blocks<S, COL_BGK_SMAG>()
                                                                           : direct_min_blocks<S, COL_BGK>());
     a.release_row = (int)(rows - (wave + per_row - 1) / per_row);
+    a.first_plane = first;
+    a.keep = keep ? 1 : 0;
     a.sr_seed = sr_step_seed(t);
     return a;
   }
@@ -72,10 +74,12 @@ struct Launchers {
     int bx = (d.L[0] + 31) / 32 * 32;
     return dim3(bx < DIRECT_BLOCK ? bx : DIRECT_BLOCK, 1, 1);
   }
-  static dim3 grid_dim(const DeviceState &d) {
+  static dim3 grid_dim(const DeviceState &d, int planes) {
     const int bx = (int)block_dim(d).x;
-    return dim3((unsigned)((d.L[0] + bx - 1) / bx), (unsigned)d.L[1], (unsigned)d.L[2]);
+    const unsigned nx = (unsigned)((d.L[0] + bx - 1) / bx);
+    return d.dim == 3 ? dim3(nx, (unsigned)d.L[1], (unsigned)planes) : dim3(nx, (unsigned)planes, 1);
   }
+  static dim3 grid_dim(const DeviceState &d) { return grid_dim(d, plane_count(d)); }
   static long long blocks(const DeviceState &d) {
     const dim3 g = grid_dim(d);
     return (long long)g.x * g.y * g.z;
@@ -99,7 +103,7 @@ struct Launchers {
   }
 
   template <int COL, bool FORCE, bool BLEND, bool DIAG>
-  static cudaError_t launch(const StepArgs<C> &a, const DeviceState &d, cudaStream_t st) {
+  static cudaError_t launch(const StepArgs<C> &a, const DeviceState &d, int planes, cudaStream_t st) {
     // The learned closure evaluates its network warp-wide, which the direct
     // kernel's converged warps allow: it never runs in the pipelined kernel.
     if constexpr (!learned_closure(COL)) {
@@ -116,7 +120,7 @@ struct Launchers {
         return cudaSuccess;
       }
     }
-    auto run = [&](auto kern) { return launch_chained(kern, grid_dim(d), block_dim(d), st, a); };
+    auto run = [&](auto kern) { return launch_chained(kern, grid_dim(d, planes), block_dim(d), st, a); };
     if (!d.aa) return run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_SHIFT>);
     if (d.tiled)
       return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_ODD>)
@@ -126,24 +130,24 @@ struct Launchers {
   }
 
   template <int COL, bool BLEND>
-  static cudaError_t launch_fd(const StepArgs<C> &a, const DeviceState &d, bool diag, cudaStream_t st) {
+  static cudaError_t launch_fd(const StepArgs<C> &a, const DeviceState &d, bool diag, int planes, cudaStream_t st) {
     if (d.forcing) {
-      if (diag) return launch<COL, true, BLEND, true>(a, d, st);
-      return launch<COL, true, BLEND, false>(a, d, st);
+      if (diag) return launch<COL, true, BLEND, true>(a, d, planes, st);
+      return launch<COL, true, BLEND, false>(a, d, planes, st);
     }
-    if (diag) return launch<COL, false, BLEND, true>(a, d, st);
-    return launch<COL, false, BLEND, false>(a, d, st);
+    if (diag) return launch<COL, false, BLEND, true>(a, d, planes, st);
+    return launch<COL, false, BLEND, false>(a, d, planes, st);
   }
 
   template <int COL>
-  static cudaError_t launch_col(const StepArgs<C> &a, const DeviceState &d, bool diag, cudaStream_t st) {
-    if (d.blend) return launch_fd<COL, true>(a, d, diag, st);
-    return launch_fd<COL, false>(a, d, diag, st);
+  static cudaError_t launch_col(const StepArgs<C> &a, const DeviceState &d, bool diag, int planes, cudaStream_t st) {
+    if (d.blend) return launch_fd<COL, true>(a, d, diag, planes, st);
+    return launch_fd<COL, false>(a, d, diag, planes, st);
   }
 
-  static cudaError_t step(const DeviceState &d, long long t, bool store, bool diag,
+  static cudaError_t step(const DeviceState &d, long long t, bool store, bool diag, int first, int planes, bool keep,
                           cudaStream_t st) {
-    const StepArgs<C> a = make_args(d, t, store);
+    const StepArgs<C> a = make_args(d, t, store, first, planes, keep);
     if (d.n_sf > 0) {
       const int nb = (d.n_sf + 127) / 128;
       sf_gather_kernel<L, S><<<nb, 128, 0, st>>>(a, d.sf_nodes, d.sf_face, d.n_sf,
@@ -151,12 +155,12 @@ struct Launchers {
     }
     cudaError_t e;
     switch (d.col) {
-      case COL_BGK: e = launch_col<COL_BGK>(a, d, diag, st); break;
-      case COL_BGK_SMAG: e = launch_col<COL_BGK_SMAG>(a, d, diag, st); break;
-      case COL_MRT_NC: e = launch_col<COL_MRT_NC>(a, d, diag, st); break;
-      case COL_BGK_MLP: e = launch_col<COL_BGK_MLP>(a, d, diag, st); break;
-      case COL_BGK_MLP1: e = launch_col<COL_BGK_MLP1>(a, d, diag, st); break;
-      default: e = launch_col<COL_MRT>(a, d, diag, st); break;
+      case COL_BGK: e = launch_col<COL_BGK>(a, d, diag, planes, st); break;
+      case COL_BGK_SMAG: e = launch_col<COL_BGK_SMAG>(a, d, diag, planes, st); break;
+      case COL_MRT_NC: e = launch_col<COL_MRT_NC>(a, d, diag, planes, st); break;
+      case COL_BGK_MLP: e = launch_col<COL_BGK_MLP>(a, d, diag, planes, st); break;
+      case COL_BGK_MLP1: e = launch_col<COL_BGK_MLP1>(a, d, diag, planes, st); break;
+      default: e = launch_col<COL_MRT>(a, d, diag, planes, st); break;
     }
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
@@ -207,14 +211,14 @@ struct Launchers {
 
   static cudaError_t fetch_population(const DeviceState &d, long long t, int i, double *out,
                                       cudaStream_t st) {
-    const StepArgs<C> a = make_args(d, t, false);
+    const StepArgs<C> a = make_args(d, t, false, 0, plane_count(d), false);
     fetch_population_kernel<L, S><<<grid_dim(d), block_dim(d), 0, st>>>(a, i, out);
     return cudaGetLastError();
   }
 
   static cudaError_t upload_population(const DeviceState &d, long long t, int i, const double *in,
                                        cudaStream_t st) {
-    const StepArgs<C> a = make_args(d, t, false);
+    const StepArgs<C> a = make_args(d, t, false, 0, plane_count(d), false);
     upload_population_kernel<L, S><<<grid_dim(d), block_dim(d), 0, st>>>(a, i, in);
     return cudaGetLastError();
   }

@@ -53,10 +53,28 @@ __device__ __forceinline__ void unroll(F &&f) {
 template <class S>
 struct Storage;
 
-// Storage formats.  put() writes a population to global memory with the
-// streaming (evict-first) cache hint: every slot is written once per step and
-// next read one step later, after the whole population set has streamed
-// through the 126 MB L2.  put_any() is a plain store for pointers that may be
+// L2 policy of the population stores.  Every slot is written once per step
+// and next read one step later: where the whole population set streams
+// through the 126 MB L2 in between, it is written evict-first; where the next
+// step of a sweep follows while the planes are still in L2, evict-last.  The
+// 2-byte formats always take the streaming hint: their sweep's planes stay in
+// L2 anyway, and the policy operand costs the issue-bound step 3%.
+using L2Policy = unsigned long long;
+__device__ __forceinline__ L2Policy l2_policy(bool keep) {
+  L2Policy first, last;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(last));
+  return keep ? last : first;
+}
+__device__ __forceinline__ void store_hinted(double *p, double v, L2Policy h) {
+  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(h) : "memory");
+}
+__device__ __forceinline__ void store_hinted(float *p, float v, L2Policy h) {
+  asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(h) : "memory");
+}
+
+// Storage formats.  put() writes a population to global memory with an L2
+// policy.  put_any() is a plain store for pointers that may be
 // in shared memory (the bulk-copy pipeline's stages); the .cs hint is a
 // global-space instruction and must never see a shared-memory address.
 template <>
@@ -64,7 +82,7 @@ struct Storage<double> {
   using C = double;
   static constexpr bool SCALED = false;
   static __device__ __forceinline__ C get(const double *p) { return *p; }
-  static __device__ __forceinline__ void put(double *p, C v) { __stcs(p, v); }
+  static __device__ __forceinline__ void put(double *p, C v, L2Policy h) { store_hinted(p, v, h); }
   static __device__ __forceinline__ void put_any(double *p, C v) { *p = v; }
 };
 template <>
@@ -72,7 +90,7 @@ struct Storage<float> {
   using C = float;
   static constexpr bool SCALED = false;
   static __device__ __forceinline__ C get(const float *p) { return *p; }
-  static __device__ __forceinline__ void put(float *p, C v) { __stcs(p, v); }
+  static __device__ __forceinline__ void put(float *p, C v, L2Policy h) { store_hinted(p, v, h); }
   static __device__ __forceinline__ void put_any(float *p, C v) { *p = v; }
 };
 // FP16 keeps (f - w) * scale so that small deviations stay out of the
@@ -82,7 +100,9 @@ struct Storage<__half> {
   using C = float;
   static constexpr bool SCALED = true;
   static __device__ __forceinline__ C get(const __half *p) { return __half2float(*p); }
-  static __device__ __forceinline__ void put(__half *p, C v) { __stcs(p, __float2half_rn(v)); }
+  static __device__ __forceinline__ void put(__half *p, C v, L2Policy) {
+    __stcs(reinterpret_cast<unsigned short *>(p), __half_as_ushort(__float2half_rn(v)));
+  }
   static __device__ __forceinline__ void put_any(__half *p, C v) { *p = __float2half_rn(v); }
 };
 // FP16 written with stochastic rounding (LBMC_F16_SR): the same 2-byte
@@ -102,7 +122,7 @@ struct Storage<half_sr> {
   using C = float;
   static constexpr bool SCALED = true;
   static __device__ __forceinline__ C get(const half_sr *p) { return __half2float(__ushort_as_half(p->bits)); }
-  static __device__ __forceinline__ void put(half_sr *p, C v) {
+  static __device__ __forceinline__ void put(half_sr *p, C v, L2Policy) {
     __stcs(reinterpret_cast<unsigned short *>(p), __half_as_ushort(__float2half_rn(v)));
   }
   static __device__ __forceinline__ void put_any(half_sr *p, C v) { p->bits = __half_as_ushort(__float2half_rn(v)); }
@@ -116,7 +136,9 @@ struct Storage<__nv_bfloat16> {
   using C = float;
   static constexpr bool SCALED = false;
   static __device__ __forceinline__ C get(const __nv_bfloat16 *p) { return __bfloat162float(*p); }
-  static __device__ __forceinline__ void put(__nv_bfloat16 *p, C v) { __stcs(p, __float2bfloat16_rn(v)); }
+  static __device__ __forceinline__ void put(__nv_bfloat16 *p, C v, L2Policy) {
+    __stcs(p, __float2bfloat16_rn(v));
+  }
   static __device__ __forceinline__ void put_any(__nv_bfloat16 *p, C v) { *p = __float2bfloat16_rn(v); }
 };
 
@@ -147,11 +169,11 @@ __device__ __forceinline__ typename Storage<S>::C load_dev(const S *p, typename 
     return Storage<S>::get(p);
   }
 }
-// Global-memory population store (streaming hint).
+// Global-memory population store.
 template <class S>
-__device__ __forceinline__ void store_dev(S *p, typename Storage<S>::C v, typename Storage<S>::C scale) {
-  if constexpr (Storage<S>::SCALED) Storage<S>::put(p, v * scale);
-  else Storage<S>::put(p, v);
+__device__ __forceinline__ void store_dev(S *p, typename Storage<S>::C v, typename Storage<S>::C scale, L2Policy h) {
+  if constexpr (Storage<S>::SCALED) Storage<S>::put(p, v * scale, h);
+  else Storage<S>::put(p, v, h);
 }
 // Shared-memory (or generic) population store, no cache hint.
 template <class S>
@@ -338,6 +360,8 @@ struct StepArgs {
   const uint16_t *table;        // 256 class-table entries (device memory)
   const MlpStep *closure;       // learned closure (COL_BGK_MLP, COL_BGK_MLP1): weights
   MlpConsts mlp;                // and its scalars
+  int first_plane;              // direct kernel: plane of block row 0 (z in 3-D, y in 2-D)
+  int keep;                     // direct kernel: the next step follows while the planes are in L2
   int release_row;              // direct kernel: block rows from here on release the next step
   unsigned sr_seed;             // stochastic-rounding seed of this step (sr_step_seed(t))
 };
@@ -1238,6 +1262,11 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   constexpr int Q = L::Q;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = x < a.L[0];
+  // The grid covers whole planes from first_plane on, past the last one from
+  // plane 0 again.
+  int cy = blockIdx.y, cz = blockIdx.z;
+  if constexpr (L::DIM == 3) cz = wrap_add(cz, a.first_plane, a.L[2]);
+  else cy = wrap_add(cy, a.first_plane, a.L[1]);
   // Read slot of population i: (i, slot(i)) in the shift layout, (i, n) at
   // an AA-even step, (opp(i), slot(i)) with the t = 1 shift at an AA-odd
   // step; out[i] goes back to slot(i) (shift) or to population opp(i)'s
@@ -1254,11 +1283,11 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   // the sites instead of keeping them live (the learned closure's stores).
   auto init_sites = [&](Sites &st, TiledSites &ts, int zero = 0) {
     if constexpr (STREAM == STREAM_AAT_EVEN)
-      ts.init_even(blockIdx.x + zero, threadIdx.x, blockIdx.y, blockIdx.z, a.L, Q);
+      ts.init_even(blockIdx.x + zero, threadIdx.x, cy, cz, a.L, Q);
     else if constexpr (STREAM == STREAM_AAT_ODD)
-      ts.init_odd(blockIdx.x + zero, threadIdx.x, blockIdx.y, blockIdx.z, a.s, a.L, Q);
+      ts.init_odd(blockIdx.x + zero, threadIdx.x, cy, cz, a.s, a.L, Q);
     else if constexpr (STREAM != STREAM_AA_EVEN)
-      st.init(x + zero, blockIdx.y, blockIdx.z, a.s, a.L);
+      st.init(x + zero, cy, cz, a.s, a.L);
   };
   double dv[DIAG_VALUES] = {0, 0, 0, 0, 0};
   bool nonfinite = false;
@@ -1277,7 +1306,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       Sites st;
       TiledSites ts;
       init_sites(st, ts);
-      const int n = x + a.L[0] * ((int)blockIdx.y + a.L[1] * (int)blockIdx.z);
+      const int n = x + a.L[0] * (cy + a.L[1] * cz);
       S *f = reinterpret_cast<S *>(a.f);
       Node<L, C> nd;
       wait_for_predecessor();
@@ -1307,7 +1336,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
         else if constexpr (std::is_same<S, __half>::value)
           store_node_f16<Q>(out, scale, [&](auto ic) { return write_at(f, sw, tw, n, ic); });
         else
-          unroll<Q>([&](auto ic) { store_dev(write_at(f, sw, tw, n, ic), out[decltype(ic)::value], scale); });
+          unroll<Q>([&](auto ic) { store_dev(write_at(f, sw, tw, n, ic), out[decltype(ic)::value], scale, l2_policy(a.keep)); });
       };
       if constexpr (recompute) {
         TiledSites tw = ts;
@@ -1331,7 +1360,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       const C inv_scale = a.inv_scale, scale = a.scale;
       Sites st;
       TiledSites ts;
-      const int n = active ? x + a.L[0] * ((int)blockIdx.y + a.L[1] * (int)blockIdx.z) : 0;
+      const int n = active ? x + a.L[0] * (cy + a.L[1] * cz) : 0;
       S *f = reinterpret_cast<S *>(a.f);
       Node<L, C> nd;
       wait_for_predecessor();
@@ -1365,7 +1394,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
           store_node_sr<Q, true>(out, scale, (unsigned)n ^ a.sr_seed,
                                  [&](auto ic) { return write_at(f, sw, tw, n, ic); });
         else
-          unroll<Q>([&](auto ic) { store_dev(write_at(f, sw, tw, n, ic), out[decltype(ic)::value], scale); });
+          unroll<Q>([&](auto ic) { store_dev(write_at(f, sw, tw, n, ic), out[decltype(ic)::value], scale, l2_policy(a.keep)); });
         store_and_reduce(nd, a, n, dv, nonfinite, DIAG);
       }
     }
@@ -1709,7 +1738,7 @@ __global__ void upload_population_kernel(const StepArgs<typename Storage<S>::C> 
   S *f = reinterpret_cast<S *>(a.f);
   unroll<L::Q>([&](auto kc) {
     constexpr int k = decltype(kc)::value;
-    if (k == i) store_dev(f + natural_slot<L, k>(a, st), (C)(in[n] - weight<L>(k)), a.scale);
+    if (k == i) store_dev(f + natural_slot<L, k>(a, st), (C)(in[n] - weight<L>(k)), a.scale, l2_policy(false));
   });
 }
 
