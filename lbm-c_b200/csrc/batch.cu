@@ -14,14 +14,16 @@
 //   - one block per domain, K steps per launch (the same persistent kernel
 //     without the shared-memory copy): a domain's K steps run back to back,
 //     so a 2-byte domain of moderate size is re-read from cache;
-//   - over every SM, one step per launch (batch_wide_kernel: one warp per
-//     segment of consecutive nodes, every listed domain in one launch),
-//     followed by a one-thread-per-domain kernel (batch_wide_finish_kernel)
-//     for the convergence test and step accounting.  Large domains need the
-//     most steps and would otherwise finish last on one SM each.
-// One CUDA graph launch holds the shared-memory kernel in one branch and the
-// block-stepped kernel followed by K wide step pairs in the other.  Every C
-// steps a domain compares u with its value C steps earlier (max norm) and
+//   - over every SM, one step per launch (batch_wide_kernel, one for even and
+//     one for odd steps: one warp per segment of consecutive nodes, every
+//     listed domain in one launch), with a one-thread-per-domain kernel
+//     (batch_wide_finish_kernel) after the steps that test for convergence
+//     and after the last one.  Large domains need the most steps and would
+//     otherwise finish last on one SM each.
+// One CUDA graph launch holds the shared-memory kernel, the block-stepped
+// kernel and the K wide steps in three branches.  Every running domain has
+// taken the same number of steps (a domain that stopped is frozen for good),
+// so the host knows each launch's step counter.  Every C steps a domain compares u with its value C steps earlier (max norm) and
 // freezes once below the tolerance, recording the device timer.  The host
 // replays the graph until every domain converged, stopped or hit the step
 // cap.  Once fewer than wide_below block-stepped domains run, they join the
@@ -43,6 +45,7 @@
 #include "../../include/lbmc.h"
 #include "engine_internal.h"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 using namespace lbmc;
 
@@ -93,18 +96,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// One D2Q9 node in the AA pattern (one array per population, in place;
-// 2-byte storage, see batch_aa below):
+// One D2Q9 node in the AA pattern (one array per population, in place):
 // at an even step the node reads population i from its own slot of array i
 // and writes out[i] to its own slot of array opp(i); at an odd step it reads
 // population i from array opp(i) at x - e_i and writes out[i] to array i at
 // x + e_i (periodic wrap).  A node writes exactly the slots it read, so the
-// update is race-free in place, and the state after every step equals the
-// shift layout's up to where the values sit (the single-domain engine's
-// LBMC_STREAM_AA maps).  Collide, write back; returns u = j/rho + F/(2 rho)
-// in `u` (the stored velocity of LBM-C/collision.cu:77).
+// update is race-free in place (the single-domain engine's LBMC_STREAM_AA
+// maps).  Collide, write back; returns u = j/rho + F/(2 rho) in `u` (the
+// stored velocity of LBM-C/collision.cu:77).
 template <class S, bool BLEND, bool ODD>
-__device__ __forceinline__ void batch_node_aa(S *pop, long long pitch, int k, int x, int y, int lx, int ly,
+__device__ __forceinline__ void batch_node(S *pop, long long pitch, int k, int x, int y, int lx, int ly,
                                               int cls, const StepArgs<float> &a, float &ux, float &uy) {
   using L = D2Q9;
   int xs[3] = {x, x, x}, ys[3] = {y, y, y};
@@ -152,67 +153,6 @@ __device__ __forceinline__ void batch_node_aa(S *pop, long long pitch, int k, in
   }
   ux = nd.u[0];
   uy = nd.u[1];
-}
-
-// One D2Q9 node: load its 9 shift slots from `pop` (pitch elements apart),
-// collide, write back; returns u = j/rho + F/(2 rho) in `u` (the stored
-// velocity of LBM-C/collision.cu:77).
-template <class S, bool BLEND>
-__device__ __forceinline__ void batch_node_shift(S *pop, long long pitch, int k, int x, int y, int lx, int ly,
-                                                 int sx, int sy, int cls, const StepArgs<float> &a,
-                                                 float &ux, float &uy) {
-  using L = D2Q9;
-  const int xs[3] = {x, wrap_sub(x, sx, lx), wrap_add(x, sx, lx)};
-  const int ys[3] = {y, wrap_sub(y, sy, ly), wrap_add(y, sy, ly)};
-  Node<L, float> nd;
-  unroll<9>([&](auto ic) {
-    constexpr int i = decltype(ic)::value;
-    const int slot = xs[sel(L::e(0, i))] + lx * ys[sel(L::e(1, i))];
-    nd.g[i] = load_dev(pop + i * pitch + slot, a.inv_scale);
-  });
-  float out[9];
-  if (cls == CLASS_SOLID) {
-    collide_solid(nd, out);
-  } else {
-    moments(nd);
-    // a.B is this domain's porosity array; only partial nodes read it.
-    collide_fluid<L, float, COL_BGK, true, BLEND, true>(nd, a, k, cls == 2 ? ENTRY_PARTIAL : 0u, out);
-  }
-  // The store slots equal the load slots; recomputing them from the six
-  // coordinates is cheaper than keeping nine addresses live across the
-  // collision (the empty asm hides the equality from the compiler).
-  int xw[3] = {xs[0], xs[1], xs[2]}, yw[3] = {ys[0], ys[1], ys[2]};
-  asm("" : "+r"(xw[0]), "+r"(xw[1]), "+r"(xw[2]), "+r"(yw[0]), "+r"(yw[1]), "+r"(yw[2]));
-  unroll<9>([&](auto ic) {
-    constexpr int i = decltype(ic)::value;
-    const int slot = xw[sel(L::e(0, i))] + lx * yw[sel(L::e(1, i))];
-    store_smem(pop + i * pitch + slot, out[i], a.scale);
-  });
-  ux = nd.u[0];
-  uy = nd.u[1];
-}
-
-// The layout of the batched domains, per storage format.  Measured on the
-// 4096-domain sweep (first 20,000 steps, one B200): 2-byte storage 80.1
-// GLUPS in the shift layout, 84.9 in the AA pattern; FP32 55.4 shift, 51.1-53.9
-// AA (its wide kernel, which FP16 does not use by default, holds both AA
-// maps and spills or loses occupancy at its register cap).
-template <class S>
-__host__ __device__ constexpr bool batch_aa() {
-  return sizeof(S) == 2;
-}
-
-// The step of node k at step t: shift t mod (lx, ly) or AA parity t & 1.
-template <class S, bool BLEND>
-__device__ __forceinline__ void batch_node(S *pop, long long pitch, int k, int x, int y, int lx, int ly,
-                                           int sx, int sy, bool odd, int cls, const StepArgs<float> &a,
-                                           float &ux, float &uy) {
-  if constexpr (batch_aa<S>()) {
-    if (odd) batch_node_aa<S, BLEND, true>(pop, pitch, k, x, y, lx, ly, cls, a, ux, uy);
-    else batch_node_aa<S, BLEND, false>(pop, pitch, k, x, y, lx, ly, cls, a, ux, uy);
-  } else {
-    batch_node_shift<S, BLEND>(pop, pitch, k, x, y, lx, ly, sx, sy, cls, a, ux, uy);
-  }
 }
 
 // The convergence measure keeps a non-finite velocity visible: fmaxf
@@ -298,7 +238,6 @@ __global__ void __launch_bounds__(1024) batch_kernel(const BatchArgs A) {
     long long t = st.t;
     int stop = 0;
     for (int s = 0; s < A.steps && !stop; s++, t++) {
-      const int sx = batch_aa<S>() ? 0 : (int)(t % D.lx), sy = batch_aa<S>() ? 0 : (int)(t % D.ly);
       const bool odd = t & 1;
       // Every C steps: du = max |u(t) - u(t - C)|, then u(t) is kept for the
       // next check.  Reduced-precision dynamics that settle into a fixed point
@@ -312,7 +251,8 @@ __global__ void __launch_bounds__(1024) batch_kernel(const BatchArgs A) {
       for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const int c = cls[k];
         float ux, uy;
-        batch_node<S, BLEND>(pop, pitch, k, x, y, D.lx, D.ly, sx, sy, odd, c, a, ux, uy);
+        if (odd) batch_node<S, BLEND, true>(pop, pitch, k, x, y, D.lx, D.ly, c, a, ux, uy);
+        else batch_node<S, BLEND, false>(pop, pitch, k, x, y, D.lx, D.ly, c, a, ux, uy);
         if (test) dmax = nan_max(dmax, node_delta(ux, uy, up[k]));
         if (save) up[k] = make_float2(ux, uy);
         x += step_x;
@@ -358,41 +298,35 @@ __global__ void __launch_bounds__(1024) batch_kernel(const BatchArgs A) {
 __global__ void stamp_kernel(unsigned long long *out) { *out = global_ns(); }
 
 // Wide phase: one step of the listed HBM domains per launch over every SM.
-// The work is cut into segments of WIDE_ITERS x 32 consecutive nodes of a
-// domain (node index k = x + lx y), one per warp, two warps per block, one
-// block per two segments; a warp loads a segment's descriptors once and
-// steps 32 nodes per iteration.  A segment records the (x, y) of its first
-// node; a lane adds its offset to x and wraps into the next row when x
-// passes lx, so no node index is divided, and only the last segment of a
-// domain has idle lanes.
+// The work is cut into segments of 32 consecutive nodes of a domain (node
+// index k = x + lx y), one per warp, two warps per block.  A segment's record
+// holds all that its warp needs (one level of dependent loads before the
+// populations), with the (x, y) of its first node: a lane adds its offset to
+// x and wraps into the next row when x passes lx, so no node index is
+// divided, and only the last segment of a domain has idle lanes.
 // The convergence test's warp maxima go to acc[domain] (non-negative
 // floats compare as their bit patterns, and the positive NaN of a
 // non-finite velocity is above every one of them).
+//
+// Even and odd steps are kernels of their own: one kernel with both maps
+// spilled at this occupancy, and the even step needs no coordinates.  The
+// steps are chained (launch.cuh), and the per-domain kernel runs after the
+// steps that test and after the last one only.  WIDE_MEASURED
 constexpr int WIDE_THREADS = 64;
 constexpr int WIDE_WARPS = WIDE_THREADS / 32;
-constexpr int WIDE_ITERS = 1;  // a segment is WIDE_ITERS x 32 consecutive nodes, one warp's work
-struct RowSegment {
-  int domain, y, x0;  // first node (x0, y) of the segment
-};
-// What the next step of a listed domain needs, prepared once per domain and
-// step (by the host when the list is built, then by the finish kernel), so
-// that no warp divides the 64-bit step counter: the shift t mod (lx, ly),
-// the parity of t (AA) and the flags below.
-struct WideStep {
-  int sx, sy;
-  int flags;
-};
-constexpr int WIDE_RUNNING = 1, WIDE_SAVE = 2, WIDE_TEST = 4, WIDE_ODD = 8;
-
-__host__ __device__ inline WideStep wide_step(long long t, int lx, int ly, int check, bool running) {
-  WideStep w;
-  w.sx = (int)(t % lx);
-  w.sy = (int)(t % ly);
-  const bool save = (t % check) == 0;
-  w.flags = (running ? WIDE_RUNNING : 0) | (save ? WIDE_SAVE : 0) | (save && t >= check ? WIDE_TEST : 0) |
-            ((t & 1) ? WIDE_ODD : 0);
-  return w;
+// Resident blocks per SM: the even step fits the register cap of 20 blocks
+// (48), the odd one spills 40 bytes there and none at 18 (56).
+template <bool ODD>
+constexpr int wide_min_blocks() {
+  return ODD ? 18 : 20;
 }
+struct __align__(16) WideSegment {
+  long long pop, node;  // the domain's populations in the pool, its nodes in cls / B / u_prev
+  int pitch, n;         // elements between populations, nodes of the domain
+  int lx, ly;
+  int k0, x0, y0;       // first node of the segment
+  int domain;
+};
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -400,23 +334,18 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Resident blocks of the wide kernel per SM: the register cap of 20 blocks
-// (48 registers) holds the shift step; the AA step (both maps in one kernel)
-// spills 28-76 bytes there and 0-24 at 18 blocks (56 registers).
-template <class S>
-constexpr int wide_min_blocks() {
-  return batch_aa<S>() ? 18 : 20;
-}
-
-template <class S, bool BLEND>
-__global__ void __launch_bounds__(WIDE_THREADS, (wide_min_blocks<S>()))
-    batch_wide_kernel(const BatchArgs A, const RowSegment *segs, int nsegs, const WideStep *steps, int *acc) {
+// save: u is kept for the next test; test: it is compared with the one kept.
+template <class S, bool BLEND, bool ODD>
+__global__ void __launch_bounds__(WIDE_THREADS, wide_min_blocks<ODD>())
+    batch_wide_kernel(const BatchArgs A, const WideSegment *segs, int nsegs, const int *running, int *acc, bool save,
+                      bool test, int release_from) {
+  if ((int)blockIdx.x >= release_from) release_successor();
   const int si = blockIdx.x * WIDE_WARPS + (int)(threadIdx.x >> 5);
-  if (si >= nsegs) return;  // whole warps
-  const RowSegment G = segs[si];
-  const WideStep W = steps[G.domain];
-  if (!(W.flags & WIDE_RUNNING)) return;  // warp-uniform: one domain per segment
-  S *pool = reinterpret_cast<S *>(A.pool);
+  const int lane = (int)(threadIdx.x & 31);
+  const WideSegment G = segs[si < nsegs ? si : nsegs - 1];
+  wait_for_predecessor();
+  if (si >= nsegs) return;          // whole warps
+  if (!running[G.domain]) return;  // warp-uniform: one domain per segment
   StepArgs<float> a;
   memset(&a, 0, sizeof(a));
   a.tau = A.tau;
@@ -430,52 +359,45 @@ __global__ void __launch_bounds__(WIDE_THREADS, (wide_min_blocks<S>()))
   a.force_u[1] = A.force[1];
   a.scale = A.scale;
   a.inv_scale = A.inv_scale;
-  const BatchDomainDev D = A.dom[G.domain];
-  const int sx = W.sx, sy = W.sy;
-  const bool odd = W.flags & WIDE_ODD;
-  const bool save = W.flags & WIDE_SAVE;
-  const bool test = W.flags & WIDE_TEST;
-  a.B = A.B + D.node_off;
-  const int lane = (int)(threadIdx.x & 31);
-  int x = G.x0 + lane, y = G.y;
-  while (x >= D.lx) {  // at most once when lx >= 32
-    x -= D.lx;
-    y += 1;
-  }
+  a.B = A.B + G.node;
+  const int k = G.k0 + lane;
   float dmax = 0;
-  float2 *up = A.u_prev + D.node_off;
-  for (int j = 0; j < WIDE_ITERS; j++) {
-    if (y >= D.ly) break;  // past the domain's last node
-    const int k = x + y * D.lx;
+  if (k < G.n) {
+    int x = G.x0 + lane, y = G.y0;
+    if constexpr (ODD) {
+      while (x >= G.lx) {  // at most once when lx >= 32
+        x -= G.lx;
+        y += 1;
+      }
+    }
     float ux, uy;
-    batch_node<S, BLEND>(pool + D.pop_off, D.pitch, k, x, y, D.lx, D.ly, sx, sy, odd, A.cls[D.node_off + k], a,
-                         ux, uy);
-    if (test) dmax = nan_max(dmax, node_delta(ux, uy, up[k]));
-    if (save) up[k] = make_float2(ux, uy);
-    x += 32;
-    while (x >= D.lx) {
-      x -= D.lx;
-      y += 1;
+    batch_node<S, BLEND, ODD>(reinterpret_cast<S *>(A.pool) + G.pop, G.pitch, k, x, y, G.lx, G.ly,
+                              A.cls[G.node + k], a, ux, uy);
+    if (save) {
+      float2 *up = A.u_prev + G.node + k;
+      if (test) dmax = node_delta(ux, uy, *up);
+      *up = make_float2(ux, uy);
     }
   }
   if (test) {
     const float m = warp_max(dmax);
-    if ((threadIdx.x & 31) == 0) atomicMax(acc + G.domain, __float_as_int(m));
+    if (lane == 0) atomicMax(acc + G.domain, __float_as_int(m));
   }
 }
 
-// After each tail-phase step: per domain, the convergence test of the step
-// just taken (max |u(t) - u(t - C)| < tol), t + 1, the step cap; at the last
-// step of a launch group the domains still running are counted.
-__global__ void batch_wide_finish_kernel(const BatchArgs A, const int *wide, int nwide, WideStep *steps, int *acc,
-                                         int last) {
+// After a step that tested, and after a launch group's last step: per listed
+// domain, the steps taken since the last call, the convergence test
+// (max |u(t) - u(t - C)| < tol) and, with `cap`, the step cap; at the last
+// step the domains still running are counted.
+__global__ void batch_wide_finish_kernel(const BatchArgs A, const int *wide, int nwide, int *running, int *acc,
+                                         int steps, bool test, bool cap, bool last) {
+  release_successor();
+  wait_for_predecessor();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nwide) return;
   const int d = wide[i];
+  if (!running[d]) return;
   BatchStateDev &st = A.state[d];
-  if (st.converged) return;
-  long long t = st.t;
-  const bool test = steps[d].flags & WIDE_TEST;
   int stop = 0;
   if (test) {
     const float m = __int_as_float(acc[d]);
@@ -483,12 +405,10 @@ __global__ void batch_wide_finish_kernel(const BatchArgs A, const int *wide, int
     st.delta_u = m;
     stop = stop_code(m, A.tol);
   }
-  t += 1;
-  if (!stop && t >= A.max_steps) stop = STOP_CAP;
-  st.t = t;
-  const BatchDomainDev D = A.dom[d];
-  steps[d] = wide_step(t, D.lx, D.ly, A.check, !stop);
+  if (!stop && cap) stop = STOP_CAP;
+  st.t += steps;
   if (stop) {
+    running[d] = 0;
     st.converged = stop;
     st.done_ns = global_ns();
   } else if (last) {
@@ -529,8 +449,9 @@ struct lbmc_batch {
   int sms = 0;
   int threads = 0, steps = 0;  // tuned launch shape
   int hbm_blocks_per_sm[3] = {1, 1, 1};  // for 256 / 512 / 1024 threads
-  cudaStream_t side = nullptr;            // second graph branch
-  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaStream_t side = nullptr, blocks = nullptr;  // graph branches of the wide steps, the block-stepped domains
+  cudaEvent_t fork = nullptr, join = nullptr, join_blocks = nullptr;
+  long long t = 0;                        // steps that every running domain has taken
   double scale = 1;
 };
 
@@ -598,32 +519,33 @@ BatchArgs make_args(lbmc_batch *b, int steps, int check, double tol, long long m
   return A;
 }
 
-// The wide domains still running, as node segments, with their step
-// descriptors (device arrays; release() frees them).
+// The wide domains still running, as node segments (device arrays; release()
+// frees them).
 struct WideWork {
-  RowSegment *segs = nullptr;
+  WideSegment *segs = nullptr;
   int *wide = nullptr;
-  WideStep *steps = nullptr;  // per domain (every domain, listed or not)
+  int *running = nullptr;  // per domain (every domain, listed or not)
   int nsegs = 0, nwide = 0;
   void release() {
     if (segs) cudaFree(segs);
     if (wide) cudaFree(wide);
-    if (steps) cudaFree(steps);
+    if (running) cudaFree(running);
     segs = nullptr;
     wide = nullptr;
-    steps = nullptr;
+    running = nullptr;
     nsegs = nwide = 0;
   }
 };
 
-// One graph launch: the resident kernel on st; on the side stream the
-// block-stepped kernel (unless its domains moved to the wide path) and then
-// K wide steps; joined again.
+// One graph launch from step counter t on, in three branches: the resident
+// kernel on st, the block-stepped kernel (unless its domains moved to the wide
+// path) and the wide steps on streams of their own; joined again.
 template <class S>
-cudaError_t launch_round(lbmc_batch *b, const BatchArgs &res, const BatchArgs &blk, const BatchArgs &wid,
+cudaError_t launch_round(lbmc_batch *b, const BatchArgs &res, const BatchArgs &blk, const BatchArgs &wid, long long t,
                          int threads, bool run_block, const WideWork &w, cudaStream_t st) {
   cudaError_t e = cudaEventRecord(b->fork, st);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(b->side, b->fork, 0);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(b->blocks, b->fork, 0);
   if (e != cudaSuccess) return e;
   if (res.ndomains > 0) {
     auto kr = b->blend ? batch_kernel<S, true, true> : batch_kernel<S, false, true>;
@@ -632,20 +554,33 @@ cudaError_t launch_round(lbmc_batch *b, const BatchArgs &res, const BatchArgs &b
   if (run_block && blk.ndomains > 0) {
     const int k = threads <= 256 ? 0 : (threads <= 512 ? 1 : 2);
     auto kh = b->blend ? batch_kernel<S, true, false> : batch_kernel<S, false, false>;
-    kh<<<b->sms * b->hbm_blocks_per_sm[k], threads, 0, b->side>>>(blk);
-  }
-  if (w.nwide > 0) {
-    auto kw = b->blend ? batch_wide_kernel<S, true> : batch_wide_kernel<S, false>;
-    const unsigned grid = (unsigned)((w.nsegs + WIDE_WARPS - 1) / WIDE_WARPS);
-    for (int s = 0; s < wid.steps; s++) {
-      kw<<<grid, WIDE_THREADS, 0, b->side>>>(wid, w.segs, w.nsegs, w.steps, b->acc);
-      batch_wide_finish_kernel<<<(w.nwide + 127) / 128, 128, 0, b->side>>>(wid, w.wide, w.nwide, w.steps, b->acc,
-                                                                          s == wid.steps - 1);
-    }
+    kh<<<std::min(blk.ndomains, b->sms * b->hbm_blocks_per_sm[k]), threads, 0, b->blocks>>>(blk);
   }
   e = cudaGetLastError();
+  if (w.nwide > 0) {
+    auto even = b->blend ? batch_wide_kernel<S, true, false> : batch_wide_kernel<S, false, false>;
+    auto odd = b->blend ? batch_wide_kernel<S, true, true> : batch_wide_kernel<S, false, true>;
+    const int grid = (w.nsegs + WIDE_WARPS - 1) / WIDE_WARPS;
+    int since = 0;  // steps the finish kernel has not seen
+    for (int s = 0; s < wid.steps && e == cudaSuccess; s++) {
+      const long long ts = t + s;
+      const bool save = ts % wid.check == 0, test = save && ts >= wid.check, last = s == wid.steps - 1;
+      // only the last wave of blocks releases the next launch (see step_kernel)
+      e = launch_chained(ts & 1 ? odd : even, dim3(grid), dim3(WIDE_THREADS), b->side, wid,
+                         (const WideSegment *)w.segs, w.nsegs, (const int *)w.running, b->acc, save, test,
+                         grid - b->sms * wide_min_blocks<true>());
+      since++;
+      if (e == cudaSuccess && (test || last)) {
+        e = launch_chained(batch_wide_finish_kernel, dim3((w.nwide + 127) / 128), dim3(128), b->side, wid,
+                           (const int *)w.wide, w.nwide, w.running, b->acc, since, test, ts + 1 >= wid.max_steps, last);
+        since = 0;
+      }
+    }
+  }
   if (e == cudaSuccess) e = cudaEventRecord(b->join, b->side);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b->join, 0);
+  if (e == cudaSuccess) e = cudaEventRecord(b->join_blocks, b->blocks);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b->join_blocks, 0);
   return e;
 }
 
@@ -657,40 +592,40 @@ cudaError_t enqueue_round(lbmc_batch *b, int steps, int check, double tol, long 
   const BatchArgs blk = make_args(b, steps, check, tol, max_steps, CLASS_BLOCK);
   const BatchArgs wid = make_args(b, steps, check, tol, max_steps, CLASS_WIDE);
   switch (b->cfg.storage) {
-    case LBMC_F16: return launch_round<__half>(b, res, blk, wid, threads, run_block, w, st);
-    case LBMC_BF16: return launch_round<__nv_bfloat16>(b, res, blk, wid, threads, run_block, w, st);
-    default: return launch_round<float>(b, res, blk, wid, threads, run_block, w, st);
+    case LBMC_F16: return launch_round<__half>(b, res, blk, wid, b->t, threads, run_block, w, st);
+    case LBMC_BF16: return launch_round<__nv_bfloat16>(b, res, blk, wid, b->t, threads, run_block, w, st);
+    default: return launch_round<float>(b, res, blk, wid, b->t, threads, run_block, w, st);
   }
 }
 
-// The wide domains still running (with include_block the block-stepped ones
-// too), as node segments; device arrays in w (the caller releases them).
-cudaError_t build_wide(lbmc_batch *b, int check, bool include_block, WideWork &w) {
+// Lists the wide domains still running (with include_block the block-stepped
+// ones too) in w; the caller releases it.
+cudaError_t build_wide(lbmc_batch *b, bool include_block, WideWork &w) {
   std::vector<BatchStateDev> st(b->ndomains);
   cudaError_t e = cudaMemcpy(st.data(), b->state, b->ndomains * sizeof(BatchStateDev), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return e;
-  std::vector<RowSegment> segs;
-  std::vector<int> wide;
-  std::vector<WideStep> steps(b->ndomains, WideStep{0, 0, 0});
+  std::vector<WideSegment> segs;
+  std::vector<int> wide, running(b->ndomains, 0);
   for (int j = b->n_resident; j < b->ndomains; j++) {
     const int d = b->order[j];
     const BatchDomainDev &D = b->dom[d];
     const bool block_stepped = j < b->n_resident + b->n_block;
     if (st[d].converged || (block_stepped && !include_block)) continue;
     wide.push_back(d);
-    steps[d] = wide_step(st[d].t, D.lx, D.ly, check, true);
-    const long long n = (long long)D.lx * D.ly;
-    for (long long k0 = 0; k0 < n; k0 += 32 * WIDE_ITERS) segs.push_back({d, (int)(k0 / D.lx), (int)(k0 % D.lx)});
+    running[d] = 1;
+    const int n = D.lx * D.ly;
+    for (int k0 = 0; k0 < n; k0 += 32)
+      segs.push_back({D.pop_off, D.node_off, D.pitch, n, D.lx, D.ly, k0, k0 % D.lx, k0 / D.lx, d});
   }
   w.nsegs = (int)segs.size();
   w.nwide = (int)wide.size();
-  e = cudaMalloc(&w.segs, sizeof(RowSegment) * std::max(1, w.nsegs));
+  e = cudaMalloc(&w.segs, sizeof(WideSegment) * std::max(1, w.nsegs));
   if (e == cudaSuccess) e = cudaMalloc(&w.wide, sizeof(int) * std::max(1, w.nwide));
-  if (e == cudaSuccess) e = cudaMalloc(&w.steps, sizeof(WideStep) * b->ndomains);
+  if (e == cudaSuccess) e = cudaMalloc(&w.running, sizeof(int) * b->ndomains);
   if (e == cudaSuccess)
-    e = cudaMemcpy(w.steps, steps.data(), sizeof(WideStep) * b->ndomains, cudaMemcpyHostToDevice);
+    e = cudaMemcpy(w.running, running.data(), sizeof(int) * b->ndomains, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && w.nsegs)
-    e = cudaMemcpy(w.segs, segs.data(), sizeof(RowSegment) * w.nsegs, cudaMemcpyHostToDevice);
+    e = cudaMemcpy(w.segs, segs.data(), sizeof(WideSegment) * w.nsegs, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && w.nwide) e = cudaMemcpy(w.wide, wide.data(), sizeof(int) * w.nwide, cudaMemcpyHostToDevice);
   // Pageable copies above: make sure they landed before the side stream reads.
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -766,14 +701,11 @@ extern "C" lbmc_status lbmc_batch_init(const lbmc_batch_config *cfg, int ndomain
     }
   }
   // HBM domains with at least wide_min_nodes nodes are stepped over every
-  // SM from the start.  Defaults measured on the 4096-domain sweep (first
-  // 20000 steps, aggregate GLUPS for thresholds 1 / 32768 / 65536 / 131072 /
-  // none): FP32 52.3 / 55.4 / 54.1 / 52.0 / 50.3, FP16 66.1 / 71.2 / 74.7 /
-  // 78.2 / 80.2 (2-byte domains stepped K times by one block stay in cache).
-  // Either way the last block-stepped domains join the wide path
-  // (wide_below), which shortens the time to steady state.
-  b->wide_min_nodes = cfg->wide_min_nodes > 0 ? cfg->wide_min_nodes
-                                              : (cfg->storage == LBMC_F32 ? 32768 : LLONG_MAX);
+  // SM from the start.  WIDE_RULE
+  b->wide_min_nodes = cfg->wide_min_nodes;
+  if (b->wide_min_nodes <= 0)
+    b->wide_min_nodes = std::min(cfg->storage == LBMC_F32 ? 32768LL : LLONG_MAX,
+                                 std::max(1LL, 3 * b->total_nodes / (4 * b->sms)));
   auto klass = [&](int d) {
     const BatchDomainDev &D = b->dom[d];
     if (D.resident) return 0;
@@ -820,6 +752,8 @@ extern "C" lbmc_status lbmc_batch_init(const lbmc_batch_config *cfg, int ndomain
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->blocks, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join_blocks, cudaEventDisableTiming);
   if (e == cudaSuccess) {
     switch (cfg->storage) {
       case LBMC_F16: e = configure_batch<__half>(b); break;
@@ -857,21 +791,27 @@ extern "C" lbmc_status lbmc_batch_run(lbmc_batch *b, long long max_steps, double
     if (e != cudaSuccess) return berr(LBMC_ERR_CUDA, std::string("lbmc_batch_run: ") + cudaGetErrorString(e));
     long long block_active = 0;
     for (int j = b->n_resident; j < b->n_resident + b->n_block; j++) block_active += !st[b->order[j]].converged;
+    for (const BatchStateDev &d : st)
+      if (!d.converged) b->t = d.t;  // the same for all of them
     all_wide = b->wide_below > 0 && block_active > 0 && block_active < b->wide_below;
-    e = build_wide(b, check_every, all_wide, w);
+    e = build_wide(b, all_wide, w);
     if (e != cudaSuccess) {
       w.release();
       return berr(LBMC_ERR_CUDA, std::string("lbmc_batch_run: ") + cudaGetErrorString(e));
     }
   }
-  auto enqueue_any = [&](int steps, int threads) {
-    return enqueue_round(b, steps, check_every, tol, max_steps, threads, !all_wide, w, b->stream);
+  // Enqueues the next `steps` steps, fewer where the step cap comes first.
+  auto enqueue_any = [&](long long steps, int threads) {
+    steps = std::min(steps, max_steps - b->t);
+    return steps < 1 ? cudaSuccess
+                     : enqueue_round(b, (int)steps, check_every, tol, max_steps, threads, !all_wide, w, b->stream);
   };
 
   // Autotune the launch shape on the first launches (they are real steps).
   if (b->threads <= 0 || b->steps <= 0) {
     const int cand_threads[3] = {256, 512, 1024};
-    const int cand_steps[2] = {check_every, 4 * check_every};
+    // even, so that every launch starts at the same parity (graph replay)
+    const int cand_steps[2] = {check_every % 2 ? 2 * check_every : check_every, 4 * check_every};
     double best = -1;
     int bt = 512, bs = check_every;
     cudaEvent_t e0, e1;
@@ -886,9 +826,12 @@ extern "C" lbmc_status lbmc_batch_run(lbmc_batch *b, long long max_steps, double
         cudaEventRecord(e1, b->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) break;
+        const long long done = std::min<long long>(sp, max_steps - b->t);
+        if (done < 1) continue;  // the cap came first
+        b->t += done;
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
-        const double rate = (double)sp / ms;  // steps per ms over the whole batch
+        const double rate = (double)done / ms;  // steps per ms over the whole batch
         if (rate > best) {
           best = rate;
           bt = th;
@@ -905,10 +848,18 @@ extern "C" lbmc_status lbmc_batch_run(lbmc_batch *b, long long max_steps, double
     b->steps = bs;
   }
 
-  // Capture one launch (queue reset + the kernels of K steps) in a graph and
-  // replay it.  Once a quarter of the listed wide domains have stopped, their
-  // segments are rebuilt and the graph re-captured, so launches no longer
-  // visit them; the same when the block-stepped domains join the wide path.
+  // One launch (queue reset + the kernels of K steps) is captured in a graph
+  // and replayed.  The graph fixes the parity of each step and the steps that
+  // test, so it serves where K is even and a multiple of the check interval
+  // (the tuned ones are), after the first test; other launches, and the last
+  // one before the step cap, are enqueued as they are.  Once a quarter of the
+  // listed wide domains have stopped, their segments are rebuilt and the graph
+  // re-captured, so launches no longer visit them; the same when the
+  // block-stepped domains join the wide path.
+  auto replayable = [&]() {
+    return b->steps % 2 == 0 && b->steps % check_every == 0 && b->t >= check_every && b->t % 2 == 0 &&
+           b->t % check_every == 0 && b->t + b->steps < max_steps;
+  };
   auto capture = [&](cudaGraph_t &graph, cudaGraphExec_t &exec) -> cudaError_t {
     cudaError_t ec = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (ec != cudaSuccess) return ec;
@@ -929,15 +880,18 @@ extern "C" lbmc_status lbmc_batch_run(lbmc_batch *b, long long max_steps, double
   auto rebuild = [&]() -> cudaError_t {
     drop_graph();
     w.release();
-    cudaError_t ew = build_wide(b, check_every, all_wide, w);
-    if (ew == cudaSuccess) ew = capture(graph, exec);
-    return ew;
+    return build_wide(b, all_wide, w);
   };
-  if (e == cudaSuccess) e = capture(graph, exec);
   int counts[5] = {0, 0, 1, 0, 0};
   const long long launches_max = max_steps / std::max(1, b->steps) + 2;
   for (long long l = 0; e == cudaSuccess && counts[2] > 0 && l < launches_max; l++) {
-    e = cudaGraphLaunch(exec, b->stream);
+    if (replayable()) {
+      if (!exec) e = capture(graph, exec);
+      if (e == cudaSuccess) e = cudaGraphLaunch(exec, b->stream);
+    } else {
+      e = enqueue_any(b->steps, b->threads);
+    }
+    b->t = std::min(max_steps, b->t + b->steps);
     if (e == cudaSuccess) e = cudaMemcpyAsync(counts, b->counters, sizeof(counts), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess || counts[2] == 0) break;
@@ -995,14 +949,12 @@ __global__ void batch_fetch_kernel(const S *pop, long long pitch, int lx, int ly
   if (k >= lx * ly) return;
   using L = D2Q9;
   const int x = k % lx, y = k / lx;
-  // Shift layout: population i of node x in array i at (x - t e_i) mod L.
   // AA pattern: after an even number of steps in array i at x; after an odd
   // number in array opp(i) at x - e_i (the next, odd step's read map).
-  const bool odd = batch_aa<S>() && (t & 1);
-  const int sx = batch_aa<S>() ? (odd ? 1 : 0) : (int)(t % lx);
-  const int sy = batch_aa<S>() ? (odd ? 1 : 0) : (int)(t % ly);
-  const int xs[3] = {x, wrap_sub(x, sx % lx, lx), wrap_add(x, sx % lx, lx)};
-  const int ys[3] = {y, wrap_sub(y, sy % ly, ly), wrap_add(y, sy % ly, ly)};
+  const bool odd = t & 1;
+  const int sx = odd ? 1 % lx : 0, sy = odd ? 1 % ly : 0;
+  const int xs[3] = {x, wrap_sub(x, sx, lx), wrap_add(x, sx, lx)};
+  const int ys[3] = {y, wrap_sub(y, sy, ly), wrap_add(y, sy, ly)};
   double r = 0, jx = 0, jy = 0;
   for (int i = 0; i < 9; i++) {
     const int slot = xs[sel(L::e(0, i))] + lx * ys[sel(L::e(1, i))];
@@ -1077,6 +1029,8 @@ extern "C" lbmc_status lbmc_batch_destroy(lbmc_batch *b) {
   if (b->side) cudaStreamDestroy(b->side);
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->join) cudaEventDestroy(b->join);
+  if (b->blocks) cudaStreamDestroy(b->blocks);
+  if (b->join_blocks) cudaEventDestroy(b->join_blocks);
   delete b;
   return LBMC_OK;
 }
