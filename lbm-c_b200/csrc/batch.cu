@@ -104,9 +104,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // update is race-free in place (the single-domain engine's LBMC_STREAM_AA
 // maps).  Collide, write back; returns u = j/rho + F/(2 rho) in `u` (the
 // stored velocity of LBM-C/collision.cu:77).
-template <class S, bool BLEND, bool ODD>
-__device__ __forceinline__ void batch_node(S *pop, long long pitch, int k, int x, int y, int lx, int ly,
-                                              int cls, const StepArgs<float> &a, float &ux, float &uy) {
+// `go` is looked at once the loads are under way: false leaves the node as
+// it is.  B_GIVEN: b is the node's Porosity (else a.B is read where needed).
+template <class S, bool BLEND, bool ODD, bool B_GIVEN = false>
+__device__ __forceinline__ bool batch_node(S *pop, long long pitch, int k, int x, int y, int lx, int ly,
+                                           int cls, const StepArgs<float> &a, float &ux, float &uy, int go = 1,
+                                           float b = 0.f) {
   using L = D2Q9;
   int xs[3] = {x, x, x}, ys[3] = {y, y, y};
   if constexpr (ODD) {
@@ -125,13 +128,15 @@ __device__ __forceinline__ void batch_node(S *pop, long long pitch, int k, int x
       nd.g[i] = load_dev(pop + i * pitch + k, a.inv_scale);
     }
   });
+  if (!go) return false;
   float out[9];
   if (cls == CLASS_SOLID) {
     collide_solid(nd, out);
   } else {
     moments(nd);
     // a.B is this domain's porosity array; only partial nodes read it.
-    collide_fluid<L, float, COL_BGK, true, BLEND, true>(nd, a, k, cls == 2 ? ENTRY_PARTIAL : 0u, out);
+    collide_fluid<L, float, COL_BGK, true, BLEND, true, B_GIVEN>(nd, a, k, cls == 2 ? ENTRY_PARTIAL : 0u, out, true,
+                                                                 b);
   }
   if constexpr (ODD) {
     // The store slots equal the load slots; recomputing them from the six
@@ -153,6 +158,7 @@ __device__ __forceinline__ void batch_node(S *pop, long long pitch, int k, int x
   }
   ux = nd.u[0];
   uy = nd.u[1];
+  return true;
 }
 
 // The convergence measure keeps a non-finite velocity visible: fmaxf
@@ -311,7 +317,12 @@ __global__ void stamp_kernel(unsigned long long *out) { *out = global_ns(); }
 // Even and odd steps are kernels of their own: one kernel with both maps
 // spilled at this occupancy, and the even step needs no coordinates.  The
 // steps are chained (launch.cuh), and the per-domain kernel runs after the
-// steps that test and after the last one only.  WIDE_MEASURED
+// steps that test and after the last one only.  Bound by the latency of its
+// loads (ncu, 40 domains FP32: 240 / 338 instructions per 32 nodes in the even
+// / odd step at 46 / 54% issue activity, 30 warps per SM).  192 domains, with
+// every HBM domain wide: FP32 53.5 -> 59 GLUPS, FP16 58.5 -> 67 (against one
+// kernel with a shift or both AA maps, three levels of descriptors and the
+// per-domain kernel after every step); 128- and 256-thread blocks: no gain.
 constexpr int WIDE_THREADS = 64;
 constexpr int WIDE_WARPS = WIDE_THREADS / 32;
 // Resident blocks per SM: the even step fits the register cap of 20 blocks
@@ -344,8 +355,14 @@ __global__ void __launch_bounds__(WIDE_THREADS, wide_min_blocks<ODD>())
   const int lane = (int)(threadIdx.x & 31);
   const WideSegment G = segs[si < nsegs ? si : nsegs - 1];
   wait_for_predecessor();
-  if (si >= nsegs) return;          // whole warps
-  if (!running[G.domain]) return;  // warp-uniform: one domain per segment
+  if (si >= nsegs) return;  // whole warps
+  // Warp-uniform (one domain per segment).  FP32 fetches the flag, the class
+  // byte, the porosity and the populations together, so that none waits for
+  // another (192 domains: 57 -> 60 GLUPS); with 2-byte storage, closer to the
+  // issue limit, the instructions of that cost more (68 -> 64), so the flag is
+  // looked at first and porosity read at partial nodes only.
+  const int go = running[G.domain];
+  if (sizeof(S) == 2 && !go) return;
   StepArgs<float> a;
   memset(&a, 0, sizeof(a));
   a.tau = A.tau;
@@ -371,15 +388,19 @@ __global__ void __launch_bounds__(WIDE_THREADS, wide_min_blocks<ODD>())
       }
     }
     float ux, uy;
-    batch_node<S, BLEND, ODD>(reinterpret_cast<S *>(A.pool) + G.pop, G.pitch, k, x, y, G.lx, G.ly,
-                              A.cls[G.node + k], a, ux, uy);
+    const int cls = A.cls[G.node + k];
+    constexpr bool early = BLEND && sizeof(S) == 4;
+    const float B = early ? A.B[G.node + k] : 0.f;
+    if (!batch_node<S, BLEND, ODD, early>(reinterpret_cast<S *>(A.pool) + G.pop, G.pitch, k, x, y, G.lx, G.ly, cls, a,
+                                          ux, uy, go, B))
+      return;
     if (save) {
       float2 *up = A.u_prev + G.node + k;
       if (test) dmax = node_delta(ux, uy, *up);
       *up = make_float2(ux, uy);
     }
   }
-  if (test) {
+  if (test && go) {
     const float m = warp_max(dmax);
     if (lane == 0) atomicMax(acc + G.domain, __float_as_int(m));
   }
@@ -700,12 +721,22 @@ extern "C" lbmc_status lbmc_batch_init(const lbmc_batch_config *cfg, int ndomain
       if (c == 2) b->blend = true;
     }
   }
-  // HBM domains with at least wide_min_nodes nodes are stepped over every
-  // SM from the start.  WIDE_RULE
+  // Which domains one SM steps by itself (shared memory, or one block in HBM)
+  // and which go over every SM.  One SM's domain must not outlast the launch:
+  // it is kept to 3/4 of an SM's share of all nodes, with a floor of 2048
+  // nodes, whose step takes a block about as long (3 us) as the shortest wide
+  // launch.  Measured, GLUPS without -> with the line: 192 domains FP16 15.6
+  // -> 65, 24 FP16 40 -> 53, 40 BF16 48 -> 63; at 3/2 of the share 192 FP16
+  // ran 49.  FP32 domains also go wide from 32768 nodes up: the 4096-domain
+  // sweep ran 52.3 / 55.4 / 54.1 / 52.0 / 50.3 GLUPS for thresholds 1 / 32768 /
+  // 65536 / 131072 / none, FP16 66.1 / 71.2 / 74.7 / 78.2 / 80.2 (2-byte domains
+  // stepped K times by one block stay in cache).
+  const long long share = std::max(2048LL, 3 * b->total_nodes / (4 * b->sms));
   b->wide_min_nodes = cfg->wide_min_nodes;
-  if (b->wide_min_nodes <= 0)
-    b->wide_min_nodes = std::min(cfg->storage == LBMC_F32 ? 32768LL : LLONG_MAX,
-                                 std::max(1LL, 3 * b->total_nodes / (4 * b->sms)));
+  if (b->wide_min_nodes <= 0) {
+    b->wide_min_nodes = cfg->storage == LBMC_F32 ? std::min(32768LL, share) : share;
+    for (BatchDomainDev &D : b->dom) D.resident = D.resident && (long long)D.lx * D.ly <= share;
+  }
   auto klass = [&](int d) {
     const BatchDomainDev &D = b->dom[d];
     if (D.resident) return 0;

@@ -922,9 +922,11 @@ __device__ __forceinline__ void mrt_d3q15(const Node<D3Q15, C> &nd, const C *sra
 // Guo source from the host's per-population terms guo_a / guo_b / guo_odd.
 // The single-domain kernels keep the per-node form, whose arithmetic is the
 // same in every instantiation (shift and AA layouts, both step kernels).
-template <class L, class C, int COL, bool FORCE, bool BLEND, bool GUO_UNIFORM = false>
+// B_GIVEN: the caller has read the node's Porosity already (b_given).
+template <class L, class C, int COL, bool FORCE, bool BLEND, bool GUO_UNIFORM = false, bool B_GIVEN = false>
 __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> &a, int n,
-                                              unsigned entry, C (&out)[L::Q], bool participate = true) {
+                                              unsigned entry, C (&out)[L::Q], bool participate = true,
+                                              C b_given = C(0)) {
   constexpr int Q = L::Q;
   C B = 0;
   if (entry) {
@@ -932,7 +934,7 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
     const int micro = (entry & ENTRY_MICRO_MASK) >> ENTRY_MICRO_SHIFT;
     if (macro) apply_macro(nd, macro, a, n);
     if (micro) apply_micro(nd, micro, a, n);
-    if (BLEND && (entry & ENTRY_PARTIAL)) B = a.B[n];
+    if (BLEND && (entry & ENTRY_PARTIAL)) B = B_GIVEN ? b_given : a.B[n];
   }
   const C tau0 = a.tau;
   C F[3] = {0, 0, 0}, pre = 0, uF = 0;
