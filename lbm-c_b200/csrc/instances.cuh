@@ -59,7 +59,8 @@ struct Launchers {
     // The last blocks, as many as one wave of the chip holds, let the next
     // step come up.
     const long long per_row = grid_dim(d, planes).x, rows = (long long)planes * (d.dim == 3 ? d.L[1] : 1);
-    const long long wave = (long long)B200_SMS * (learned_closure(d.col)      ? direct_min_blocks<S, COL_BGK_MLP>()
+    const long long wave = (long long)B200_SMS * (d.col == COL_BGK_MLP1   ? direct_min_blocks<S, COL_BGK_MLP1>()
+                                                  : d.col == COL_BGK_MLP ? direct_min_blocks<S, COL_BGK_MLP>()
                                                   : d.col == COL_BGK_SMAG ? direct_min_blocks<S, COL_BGK_SMAG>()
                                                                           : direct_min_blocks<S, COL_BGK>());
     a.release_row = (int)(rows - (wave + per_row - 1) / per_row);

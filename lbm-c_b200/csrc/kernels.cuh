@@ -320,6 +320,12 @@ constexpr int STEP_BLOCK = 256;  // largest block of any step kernel
 constexpr int DIRECT_BLOCK = 64;
 constexpr int DIRECT_MIN_BLOCKS = 20;
 constexpr int DIRECT_MIN_BLOCKS_SMAG = 16;  // the Smagorinsky stress needs more registers
+// The learned closure: with the node's state in shared memory beside the
+// network, one pass fits 72 registers with 0-20 bytes of spills, the pass loop
+// 96 with 12-28.  us a step at 128^3 one pass (64^3 two passes): 8 blocks
+// with the state in registers 98 (20.5), 10 blocks 92.9 (17.0), 12 88.0
+// (17.4), 14 86.8 (17.7).
+constexpr int DIRECT_MIN_BLOCKS_MLP1 = 14, DIRECT_MIN_BLOCKS_MLP = 10;
 
 template <class C>
 struct StepArgs {
@@ -1126,18 +1132,36 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
         // warp-wide on the tensor cores, so every lane of the warp takes the
         // same number of passes (non-participating lanes feed zeros).
         __shared__ __align__(16) unsigned mlp_stage[DIRECT_BLOCK / 32][128];
+        // The node's state waits in shared memory meanwhile (one column per
+        // thread, no conflicts): held in registers beside the network it
+        // took 128 of them, 8 blocks per SM (DIRECT_MIN_BLOCKS_MLP1).
+        __shared__ C node_state[L::Q + 13][DIRECT_BLOCK];
+        auto each_state = [&](auto &&f) {
+          unroll<L::Q>([&](auto ic) { f(nd.g[decltype(ic)::value], decltype(ic)::value); });
+          unroll<3>([&](auto dc) {
+            constexpr int d = decltype(dc)::value;
+            if constexpr (d < L::DIM) {
+              f(nd.u[d], L::Q + d);
+              if constexpr (FORCE) f(F[d], L::Q + 3 + d);
+            }
+          });
+          f(nd.drho, L::Q + 6);
+        };
+        each_state([&](C &v, int k) { *(volatile C *)&node_state[k][threadIdx.x] = v; });
+        unroll<6>([&](auto cc) {
+          *(volatile C *)&node_state[L::Q + 7 + decltype(cc)::value][threadIdx.x] = q[decltype(cc)::value];
+        });
         const MlpStep *cl = a.closure;
         bool in_range = participate;
         C tau_l = tau_smag;
         // One pass for COL_BGK_MLP1 is a compile-time constant: the pass
-        // loop and what it carries disappear (128 registers, no spills,
-        // against ~163 with the runtime loop).
+        // loop and what it carries disappear.
         const int passes = COL == COL_BGK_MLP1 ? 1 : a.mlp.iterations;
         for (int it = 0; it < passes; it++) {
           const float ks = __fdividef(-1.5f, (float)(nd.rho * tau_l));
           float Sm[6], f[MLP_IN];
 #pragma unroll
-          for (int c = 0; c < 6; c++) Sm[c] = ks * (float)q[c];
+          for (int c = 0; c < 6; c++) Sm[c] = ks * (float)*(volatile C *)&node_state[L::Q + 7 + c][threadIdx.x];
           strain_features(Sm, (float)nd.rho, f);
 #pragma unroll
           for (int c = 0; c < MLP_IN; c++) {
@@ -1150,6 +1174,7 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
           if (in_range) tau_l = tau0 + C(3) * C(fmaxf(0.0f, a.mlp.target_scale * y));
         }
         tau = in_range ? tau_l : tau_smag;
+        each_state([&](C &v, int k) { v = *(volatile C *)&node_state[k][threadIdx.x]; });
       }
     }
     // 1/tau: the host's value for a uniform tau, else the local one
@@ -1251,9 +1276,10 @@ __device__ __forceinline__ void block_diag(const double (&v)[DIAG_VALUES], bool 
 // Grid: blockDim (bx, 1, 1) along x, gridDim (ceil(Lx/bx), Ly, Lz).
 template <class S, int COL>
 constexpr int direct_min_blocks() {
-  // FP64 arithmetic needs register pairs, the learned closure its hidden
-  // layer: no cap beyond the 128 per thread that 8 resident blocks imply.
-  if (std::is_same<S, double>::value || learned_closure(COL)) return 8;
+  // FP64 arithmetic needs register pairs: no cap beyond the 128 per thread
+  // that 8 resident blocks imply.
+  if (std::is_same<S, double>::value) return 8;
+  if (learned_closure(COL)) return COL == COL_BGK_MLP1 ? DIRECT_MIN_BLOCKS_MLP1 : DIRECT_MIN_BLOCKS_MLP;
   return COL == COL_BGK_SMAG ? DIRECT_MIN_BLOCKS_SMAG : DIRECT_MIN_BLOCKS;
 }
 

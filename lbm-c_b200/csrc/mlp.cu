@@ -341,14 +341,14 @@ void mlp_step_layout(const MlpClosure &cl, int iterations, MlpStep &s, MlpConsts
     const int g = lane >> 2, c = lane & 3;
     for (int j = 0; j < 4; j++) {
       const int n = 8 * j + g, k = 2 * c, col = 8 * j + 2 * c;
-      set(s.w1[lane], j, pair(k < MLP_IN ? MLP_W1 + n * MLP_IN + k : -1,
-                              k + 1 < MLP_IN ? MLP_W1 + n * MLP_IN + k + 1 : -1, 0.5f));
+      // input 6 is the constant 1 that the bias goes with
+      set(s.w1[lane], j, k < MLP_IN ? pair(MLP_W1 + n * MLP_IN + k, MLP_W1 + n * MLP_IN + k + 1, 0.5f)
+                                    : pair(MLP_B1 + n, -1, 0.5f));
       for (int kt = 0; kt < 2; kt++)
         for (int r = 0; r < 2; r++) {
           const int kk = 16 * kt + 8 * r + 2 * c;
           set(s.w2[j][lane], 2 * kt + r, pair(MLP_W2 + n * MLP_H + kk, MLP_W2 + n * MLP_H + kk + 1, 0.5f));
         }
-      set(s.b1[lane], j, pair(MLP_B1 + col, MLP_B1 + col + 1, 0.5f));
       set(s.b2[lane], j, pair(MLP_B2 + col, MLP_B2 + col + 1, 0.5f));
     }
     for (int kt = 0; kt < 2; kt++)

@@ -115,13 +115,13 @@ struct MlpConsts {
 // one coalesced 128-bit load per warp.  "pair" = two BF16 values, lower
 // column in the low half.
 struct MlpStep {
-  uint4 w1[32];      // layer 1 B fragments, N-tile j = 0..3: W1[8j+g][2c], W1[8j+g][2c+1] (halved)
+  uint4 w1[32];      // layer 1 B fragments, N-tile j = 0..3: W1[8j+g][2c], W1[8j+g][2c+1] (halved);
+                     //   for c = 3 the bias b1[8j+g] (halved) and 0: input 6 of the tile is 1
   uint4 w2[4][32];   // layer 2, N-tile j: (K-tile 0 reg 0, reg 1, K-tile 1 reg 0, reg 1),
                      //   reg r of K-tile kt: W2[8j+g][16kt+8r+2c], W2[8j+g][16kt+8r+2c+1] (halved)
   uint4 w3[32];      // layer 3 (output column 0): same order, W3[16kt+8r+2c], W3[16kt+8r+2c+1]
                      //   where g == 0, zero elsewhere
-  uint4 b1[32];      // pairs b1[8j+2c], b1[8j+2c+1] for j = 0..3 (halved)
-  uint4 b2[32];      // the same for b2
+  uint4 b2[32];      // pairs b2[8j+2c], b2[8j+2c+1] for j = 0..3 (halved)
 };
 
 // Host: the in-step form of a network (weights as BF16 bit patterns).
@@ -184,62 +184,66 @@ __device__ __forceinline__ unsigned silu_half_bf16x2(float h0, float h1) {
 // Network output without the output bias b3 (and before target_scale) for
 // the calling lane's normalised inputs.  Warp-wide: all 32 lanes call it
 // together; `stage` is this warp's 128 words of shared memory.  The two
-// 16-node tiles go through the whole network one after the other, so only
-// one tile's activations are live at a time (the step kernel keeps its
-// node state in registers meanwhile); the weight fragments of the second
-// tile are re-read from L1.
+// 16-node tiles go through each layer together, so a weight fragment is
+// loaded once for both (the step kernel parks its node state in shared memory
+// meanwhile, which leaves the registers for it).
 __device__ __forceinline__ float mlp_forward_warp(const MlpStep *__restrict__ cl,
                                                   const float (&x)[MLP_IN], unsigned *stage) {
   const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   __syncwarp();
-  // Row `lane` of the input tile: pairs (x0 x1)(x2 x3)(x4 x5)(0 0).
+  // Row `lane` of the input tile: pairs (x0 x1)(x2 x3)(x4 x5)(1 0); the 1 is
+  // layer 1's bias input.
   uint4 r4;
   r4.x = bf16x2_bits(__floats2bfloat162_rn(x[0], x[1]));
   r4.y = bf16x2_bits(__floats2bfloat162_rn(x[2], x[3]));
   r4.z = bf16x2_bits(__floats2bfloat162_rn(x[4], x[5]));
-  r4.w = 0u;
+  r4.w = 0x3f80u;
   reinterpret_cast<uint4 *>(stage)[lane] = r4;
   __syncwarp();
-  float out[4];  // entry 2t + h: tile t, row g + 8h
+  // Layer 1 -> silu_b -> layer 2's A fragments [tile][K-tile][reg].
+  unsigned a1[2][2][4], a2[2][2][4];
+  {
+    const uint4 w1 = ldg_frag(&cl->w1[lane]);
 #pragma unroll
-  for (int t = 0; t < 2; t++) {
-    const unsigned xa0 = stage[(16 * t + g) * 4 + c], xa1 = stage[(16 * t + 8 + g) * 4 + c];
-    // Layer 1 -> silu_b -> layer 2's A fragments [K-tile][reg].
-    unsigned a1[2][4];
-    {
-      const uint4 w1 = ldg_frag(&cl->w1[lane]), b1 = ldg_frag(&cl->b1[lane]);
+    for (int t = 0; t < 2; t++) {
+      const unsigned xa0 = stage[(16 * t + g) * 4 + c], xa1 = stage[(16 * t + 8 + g) * 4 + c];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const unsigned wj = u4_get(w1, j), bj = u4_get(b1, j);
         const int kt = j >> 1, r = (j & 1) * 2;  // N-tile j feeds K-tile j/2, regs r, r + 1
         float d[4];
-        mma_bf16_k8(d, xa0, xa1, wj, bf16_lo(bj), bf16_hi(bj));
-        a1[kt][r] = silu_half_bf16x2(d[0], d[1]);
-        a1[kt][r + 1] = silu_half_bf16x2(d[2], d[3]);
+        mma_bf16_k8(d, xa0, xa1, u4_get(w1, j), 0.f, 0.f);
+        a1[t][kt][r] = silu_half_bf16x2(d[0], d[1]);
+        a1[t][kt][r + 1] = silu_half_bf16x2(d[2], d[3]);
       }
     }
-    // Layer 2 -> silu_b -> layer 3's A fragments.
-    unsigned a2[2][4];
-    {
-      const uint4 b2 = ldg_frag(&cl->b2[lane]);
+  }
+  // Layer 2 -> silu_b -> layer 3's A fragments.
+  {
+    const uint4 b2 = ldg_frag(&cl->b2[lane]);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const uint4 w2 = ldg_frag(&cl->w2[j][lane]);
-        const unsigned bj = u4_get(b2, j);
-        const int kt = j >> 1, r = (j & 1) * 2;
+    for (int j = 0; j < 4; j++) {
+      const uint4 w2 = ldg_frag(&cl->w2[j][lane]);
+      const float b0 = bf16_lo(u4_get(b2, j)), b1 = bf16_hi(u4_get(b2, j));
+      const int kt = j >> 1, r = (j & 1) * 2;
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
         float d[4];
-        mma_bf16_k16_c(d, a1[0], w2.x, w2.y, bf16_lo(bj), bf16_hi(bj));
-        mma_bf16_k16(d, a1[1], w2.z, w2.w);
-        a2[kt][r] = silu_half_bf16x2(d[0], d[1]);
-        a2[kt][r + 1] = silu_half_bf16x2(d[2], d[3]);
+        mma_bf16_k16_c(d, a1[t][0], w2.x, w2.y, b0, b1);
+        mma_bf16_k16(d, a1[t][1], w2.z, w2.w);
+        a2[t][kt][r] = silu_half_bf16x2(d[0], d[1]);
+        a2[t][kt][r + 1] = silu_half_bf16x2(d[2], d[3]);
       }
     }
-    // Layer 3: column 0 of the accumulator is the output; lanes with c == 0
-    // hold rows g (d[0]) and g + 8 (d[2]).
-    const uint4 w3 = ldg_frag(&cl->w3[lane]);
+  }
+  // Layer 3: column 0 of the accumulator is the output; lanes with c == 0
+  // hold rows g (d[0]) and g + 8 (d[2]).
+  float out[4];  // entry 2t + h: tile t, row g + 8h
+  const uint4 w3 = ldg_frag(&cl->w3[lane]);
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
     float d[4];
-    mma_bf16_k16_c(d, a2[0], w3.x, w3.y, 0.f, 0.f);
-    mma_bf16_k16(d, a2[1], w3.z, w3.w);
+    mma_bf16_k16_c(d, a2[t][0], w3.x, w3.y, 0.f, 0.f);
+    mma_bf16_k16(d, a2[t][1], w3.z, w3.w);
     out[2 * t] = d[0];
     out[2 * t + 1] = d[2];
   }
