@@ -32,6 +32,7 @@
 #include "engine_internal.h"
 #include "kernels.cuh"
 #include "lattice.cuh"
+#include "launch.cuh"
 #include "mlp.cuh"
 #include "sweep.h"
 
@@ -164,6 +165,15 @@ struct HostClasses {
 
 void lbmc::set_last_error(const std::string &message) { g_last_error = message; }
 
+// What the host wants to know of a step, in page-locked host memory that the
+// last diagnostic kernel writes: valid once the stream is idle, without a
+// copy.  (Up to four blocking copies made a diagnostic step and its read-out
+// 56 + 31 us at 128x64; now 19 + 6.)
+struct Report {
+  double diag[DIAG_VALUES];
+  unsigned nonfinite;
+};
+
 struct lbmc_handle {
   lbmc_config cfg;
   DeviceState ds;
@@ -172,7 +182,8 @@ struct lbmc_handle {
   cudaStream_t own_stream = nullptr;
   long long step = 0;
   long long nblocks = 0;
-  double *diag_out = nullptr;  // DIAG_VALUES doubles
+  Report *report = nullptr;      // page-locked, written by the device
+  Report *report_dev = nullptr;  // the same, as the device sees it
   long long diag_step = -1;
   double *fetch_stage = nullptr;  // FP64 staging of uploads and lbmc_fetch (allocated on first use)
   long long fetch_stage_n = 0;
@@ -534,6 +545,7 @@ static void release(lbmc_handle *h) {
   if (!h) return;
   for (void *p : h->allocations) cudaFree(p);
   h->allocations.clear();
+  if (h->report) cudaFreeHost(h->report);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   if (h->side_stream) cudaStreamDestroy(h->side_stream);
   for (cudaEvent_t ev : {h->fork, h->join})
@@ -671,7 +683,7 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
                             sizeof(double) * stage_n,                                     // FP64 staging
                             sizeof(d.table), sizeof(unsigned),                            // table, error flag
                             sizeof(double) * DIAG_VALUES * (h->nblocks + FINALIZE_BLOCKS),  // partials
-                            sizeof(unsigned), sizeof(double) * DIAG_VALUES};              // flag, diagnostics
+                            sizeof(unsigned)};                                            // non-finite flag
     size_t total = 0;
     for (size_t b : sizes) total += (b + 255) / 256 * 256;
     char *base = nullptr;
@@ -696,8 +708,10 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
     d.error_flag = static_cast<unsigned *>(take(8));
     d.partials = static_cast<double *>(take(9));
     d.flag = static_cast<unsigned *>(take(10));
-    h->diag_out = static_cast<double *>(take(11));
   }
+  TRYCUDA(cudaHostAlloc(&h->report, sizeof(Report), cudaHostAllocMapped), "report block");
+  TRYCUDA(cudaHostGetDevicePointer(&h->report_dev, h->report, 0), "report block");
+  memset(h->report, 0, sizeof(Report));
   TRYCUDA(cudaMemsetAsync(d.error_flag, 0, sizeof(unsigned), h->stream), "clear error flag");
   TRYCUDA(cudaMemsetAsync(d.flag, 0, sizeof(unsigned), h->stream), "clear flag");
 
@@ -830,34 +844,50 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
   return LBMC_OK;
 }
 
-// Sums the per-block partials in FP64 in a fixed order (deterministic: the
-// order depends only on the number of step blocks).  Stage 1: block g of
-// FINALIZE_BLOCKS sums a contiguous run of whole partial records with
-// coalesced loads; FINALIZE_THREADS is a multiple of DIAG_VALUES, so thread
-// t always meets value t mod DIAG_VALUES, and the threads of one value are
-// then added in thread order.  Stage 2: one block adds the stage-1 sums in
-// block order.
+// Sums records of DIAG_VALUES doubles [0, n) in FP64 in a fixed order, over one
+// block of FINALIZE_THREADS threads: coalesced loads (FINALIZE_THREADS is a
+// multiple of DIAG_VALUES, so thread t always meets value t mod DIAG_VALUES),
+// then a tree over the threads of each value.  The sums are in
+// sh[0 .. DIAG_VALUES) afterwards.
+__device__ __forceinline__ void sum_records(const double *records, long long n, double *sh) {
+  double acc = 0;
+  for (long long k = threadIdx.x; k < n * DIAG_VALUES; k += FINALIZE_THREADS) acc += records[k];
+  sh[threadIdx.x] = acc;
+  __syncthreads();
+  int live = FINALIZE_THREADS / DIAG_VALUES;  // records left
+  while (live > 1) {
+    const int half = (live + 1) / 2;
+    if ((int)threadIdx.x < (live - half) * DIAG_VALUES) sh[threadIdx.x] += sh[threadIdx.x + half * DIAG_VALUES];
+    live = half;
+    __syncthreads();
+  }
+}
+
+// The block partials of a diagnostic step, summed in an order that depends
+// only on their number.  Domains of more than FINALIZE_DIRECT step blocks go
+// through a first stage: block g of FINALIZE_BLOCKS sums a contiguous run of
+// records.  The last stage, one block, hands the sums and the non-finite flag
+// to the host and clears the flag for the next time.  (A single warp that
+// added the first stage's 256 records one after the other took 13 us.)
+constexpr long long FINALIZE_DIRECT = 4096;
 __global__ void __launch_bounds__(FINALIZE_THREADS)
     diag_finalize_blocks_kernel(const double *partials, long long nblocks, double *mid) {
   __shared__ double sh[FINALIZE_THREADS];
+  wait_for_predecessor();
   const long long per = (nblocks + FINALIZE_BLOCKS - 1) / FINALIZE_BLOCKS;
-  const long long b0 = per * blockIdx.x, b1 = b0 + per < nblocks ? b0 + per : nblocks;
-  const long long end = b1 * DIAG_VALUES;
-  double acc = 0;
-  for (long long k = b0 * DIAG_VALUES + threadIdx.x; k < end; k += FINALIZE_THREADS) acc += partials[k];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.x < DIAG_VALUES) {
-    double t = 0;
-    for (int k = threadIdx.x; k < FINALIZE_THREADS; k += DIAG_VALUES) t += sh[k];
-    mid[blockIdx.x * DIAG_VALUES + threadIdx.x] = t;
-  }
+  const long long b0 = min(per * blockIdx.x, nblocks), b1 = min(b0 + per, nblocks);
+  sum_records(partials + b0 * DIAG_VALUES, b1 - b0, sh);
+  if (threadIdx.x < DIAG_VALUES) mid[blockIdx.x * DIAG_VALUES + threadIdx.x] = sh[threadIdx.x];
 }
-__global__ void diag_finalize_kernel(const double *mid, double *out) {
-  if (threadIdx.x < DIAG_VALUES) {
-    double t = 0;
-    for (int g = 0; g < FINALIZE_BLOCKS; g++) t += mid[g * DIAG_VALUES + threadIdx.x];
-    out[threadIdx.x] = t;
+__global__ void __launch_bounds__(FINALIZE_THREADS)
+    diag_finalize_kernel(const double *records, long long n, unsigned *flag, Report *report) {
+  __shared__ double sh[FINALIZE_THREADS];
+  wait_for_predecessor();
+  sum_records(records, n, sh);
+  if (threadIdx.x < DIAG_VALUES) report->diag[threadIdx.x] = sh[threadIdx.x];
+  if (threadIdx.x == 0) {
+    report->nonfinite = *flag;
+    *flag = 0;
   }
 }
 
@@ -902,29 +932,35 @@ extern "C" lbmc_status lbmc_iterate(lbmc_handle *h, int nsteps, unsigned flags) 
     const bool last = s == nsteps - 1;
     const bool store = last && (flags & LBMC_STORE_MACROS);
     const bool diag = last && (flags & LBMC_REDUCE_DIAG);
-    if (diag) CK(cudaMemsetAsync(h->ds.flag, 0, sizeof(unsigned), h->stream), "clear flag");
     CK(h->ops->step(h->ds, h->step, store, diag, 0, plane_count(h->ds), false, h->stream), "step kernel launch");
     h->step++;
     if (diag) {
-      double *mid = h->ds.partials + DIAG_VALUES * h->nblocks;
-      diag_finalize_blocks_kernel<<<FINALIZE_BLOCKS, FINALIZE_THREADS, 0, h->stream>>>(h->ds.partials,
-                                                                                       h->nblocks, mid);
-      diag_finalize_kernel<<<1, 32, 0, h->stream>>>(mid, h->diag_out);
-      CK(cudaGetLastError(), "diagnostic reduction launch");
+      const double *records = h->ds.partials;
+      long long n = h->nblocks;
+      if (n > FINALIZE_DIRECT) {
+        double *mid = h->ds.partials + DIAG_VALUES * n;
+        CK(launch_chained(diag_finalize_blocks_kernel, dim3(FINALIZE_BLOCKS), dim3(FINALIZE_THREADS), h->stream,
+                          records, n, mid),
+           "diagnostic reduction launch");
+        records = mid;
+        n = FINALIZE_BLOCKS;
+      }
+      CK(launch_chained(diag_finalize_kernel, dim3(1), dim3(FINALIZE_THREADS), h->stream, records, n, h->ds.flag,
+                        h->report_dev),
+         "diagnostic reduction launch");
       h->diag_step = h->step;
     }
   }
   if (flags & LBMC_SYNC) {
     CK(cudaStreamSynchronize(h->stream), "lbmc_iterate");
-    unsigned err = 0;
-    CK(cudaMemcpy(&err, h->ds.error_flag, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
-    if (err & ERROR_TIMEOUT)
-      return fail(LBMC_ERR_TIMEOUT, "a device-side wait expired (bulk-copy pipeline)");
-    if ((flags & LBMC_REDUCE_DIAG) && nsteps > 0) {
-      unsigned flag = 0;
-      CK(cudaMemcpy(&flag, h->ds.flag, sizeof(flag), cudaMemcpyDeviceToHost), "read flag");
-      if (flag) return fail(LBMC_ERR_NAN, "non-finite density or velocity at step %lld", h->step);
+    if (h->ds.use_pipeline) {  // the only kernel with waits that can expire
+      unsigned err = 0;
+      CK(cudaMemcpy(&err, h->ds.error_flag, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
+      if (err & ERROR_TIMEOUT)
+        return fail(LBMC_ERR_TIMEOUT, "a device-side wait expired (bulk-copy pipeline)");
     }
+    if ((flags & LBMC_REDUCE_DIAG) && nsteps > 0 && h->report->nonfinite)
+      return fail(LBMC_ERR_NAN, "non-finite density or velocity at step %lld", h->step);
   }
   return LBMC_OK;
 }
@@ -1001,17 +1037,14 @@ extern "C" lbmc_status lbmc_fetch(lbmc_handle *h, int field, void *dst, size_t b
       lbmc_diag out;
       memset(&out, 0, sizeof(out));
       if (h->diag_step >= 0) {
-        double v[DIAG_VALUES];
-        unsigned flag = 0;
-        CK(cudaMemcpy(v, h->diag_out, sizeof(v), cudaMemcpyDeviceToHost), "fetch diagnostics");
-        CK(cudaMemcpy(&flag, d.flag, sizeof(flag), cudaMemcpyDeviceToHost), "fetch diagnostics");
+        const double *v = h->report->diag;  // the stream is idle
         out.mass = v[0];
         out.momentum[0] = v[1];
         out.momentum[1] = v[2];
         out.momentum[2] = v[3];
         out.kinetic_energy = v[4];
         out.step = h->diag_step;
-        out.nonfinite = flag ? 1 : 0;
+        out.nonfinite = h->report->nonfinite ? 1 : 0;
         out.valid = 1;
       }
       memcpy(dst, &out, sizeof(out));
