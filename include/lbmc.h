@@ -138,7 +138,9 @@ typedef struct lbmc_config {
 } lbmc_config;
 
 /* Step-kernel choice (lbmc_config.kernel).  AUTO and DIRECT run the
- * direct-load kernel; PIPELINED runs the bulk-copy (TMA) row pipeline, which
+ * direct-load kernel; with AUTO, six or more steps in a row of a D2Q9 domain
+ * of at most 16384 nodes run in one launch out of shared memory (the same
+ * results).  PIPELINED runs the bulk-copy (TMA) row pipeline, which
  * needs a population row to be a whole number of 16-byte granules and two
  * shared-memory stages of Q rows to fit (else lbmc_init fails with
  * LBMC_ERR_UNSUPPORTED). */

@@ -40,6 +40,8 @@ using namespace lbmc;
 
 // Values per lbmc_fetch staging chunk (64 MiB of FP64).
 constexpr long long FETCH_CHUNK = 1ll << 23;
+// Steps that a small 2-D domain takes in one launch, at least and at most.
+constexpr int RESIDENT_MIN_STEPS = 6, RESIDENT_MAX_STEPS = 4096;
 
 namespace {
 
@@ -659,6 +661,7 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
   // and x offsets are 32-bit); other domains keep the plain AA layout.
   d.tiled = d.aa && d.L[0] % lbmc::TILE == 0 && (long long)q * n < (1ll << 32) ? 1 : 0;
   d.pipeline = cfg->kernel == LBMC_KERNEL_PIPELINED ? 2 : 0;
+  d.auto_kernel = cfg->kernel == LBMC_KERNEL_AUTO ? 1 : 0;
   TRYCUDA(h->ops->plan(d), "kernel planning");
   if (cfg->kernel == LBMC_KERNEL_PIPELINED && !d.use_pipeline) {
     release(h);
@@ -796,6 +799,7 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
   // and the bulk-copy kernel walks all rows: both go step by step.
   if (d.n_sf == 0 && !d.use_pipeline) h->sweep = plan_sweep(plane_count(d), n / plane_count(d) * q * ss, ss);
   if (h->sweep.depth > 1) TRYCUDA(make_sweep(h), "sweep streams");
+  if (d.n_sf == 0 && !d.use_pipeline) TRYCUDA(h->ops->plan_resident(d), "kernel planning");
 
   // Initial populations (Init: model_builder.cu:227-248 for Init 0).
   if (cfg->init_type == LBMC_INIT_STATIC) {
@@ -926,6 +930,15 @@ extern "C" lbmc_status lbmc_iterate(lbmc_handle *h, int nsteps, unsigned flags) 
   const int plain = nsteps - ((flags & (LBMC_STORE_MACROS | LBMC_REDUCE_DIAG)) ? 1 : 0);
   const int depth = learned_closure(h->ds.col) ? 1 : h->sweep.depth;
   int swept = 0;
+  // A small 2-D domain takes them in one cluster's shared memory, from
+  // RESIDENT_MIN_STEPS on (the launch, the load and the write-back cost ~8 us,
+  // a step 1.05 us; of the direct kernel a step costs 2.2-3.1 us), in launches
+  // of a few milliseconds.
+  if (h->ds.resident_cluster > 0 && !learned_closure(h->ds.col) && plain >= RESIDENT_MIN_STEPS)
+    for (int steps; (steps = std::min(RESIDENT_MAX_STEPS, plain - swept)) > 0; swept += steps) {
+      CK(h->ops->resident(h->ds, h->step, steps, h->stream), "step kernel launch");
+      h->step += steps;
+    }
   for (int levels; depth > 1 && (levels = std::min(depth, plain - swept)) > 1; swept += levels)
     CK(sweep(h, levels), "step kernel launch");
   for (int s = swept; s < nsteps; s++) {

@@ -47,6 +47,9 @@ struct DeviceState {
   int stages;               // shared-memory stages of the pipelined kernel
   long long pipe_grid;      // persistent blocks of the pipelined kernel
   long long nblocks;        // blocks of the step kernel (diagnostic partials)
+  int auto_kernel;          // lbmc_config.kernel leaves the choice open
+  int resident_cluster;     // blocks of the cluster that steps a small 2-D domain (0: none)
+  int resident_per;         // nodes per block of it
   void *closure;            // device MlpStep when a learned closure is attached
   lbmc::MlpConsts closure_consts;  // its scalars, passed with each launch
 };
@@ -63,6 +66,9 @@ struct LatticeStorageOps {
   // while these planes are in L2.
   cudaError_t (*step)(const DeviceState &, long long t, bool store, bool diag, int first, int planes, bool keep,
                       cudaStream_t);
+  // `steps` time steps from step counter t on in one launch (resident_cluster
+  // > 0 only; no store, no diagnostics).
+  cudaError_t (*resident)(const DeviceState &, long long t, int steps, cudaStream_t);
   // out[x] = f_i(x) in natural layout (FP64) at step counter t.
   cudaError_t (*fetch_population)(const DeviceState &, long long t, int i, double *out,
                                    cudaStream_t);
@@ -71,6 +77,9 @@ struct LatticeStorageOps {
                                    cudaStream_t);
   // Chooses the step kernel and launch geometry; sets nblocks.
   cudaError_t (*plan)(DeviceState &);
+  // Chooses the cluster that keeps a small 2-D domain in shared memory (once
+  // the classes are known); sets resident_cluster, resident_per.
+  cudaError_t (*plan_resident)(DeviceState &);
 };
 
 // Sets the calling thread's lbmc_last_error() message.

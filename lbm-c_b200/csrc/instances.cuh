@@ -13,6 +13,9 @@ namespace lbmc {
 constexpr long long PIPE_STAGE_BUDGET = 32 * 1024;
 
 constexpr int B200_SMS = 148;
+// Dynamic shared memory of a resident block at most: two buffers of 1024
+// D2Q9 nodes in FP64.
+constexpr int RESIDENT_SMEM = 2 * 9 * RESIDENT_MAX_THREADS * 8;
 
 template <class L, class S>
 struct Launchers {
@@ -167,6 +170,86 @@ struct Launchers {
     return cudaGetLastError();
   }
 
+  template <int COL, bool FORCE, bool BLEND>
+  static auto resident_kernel() {
+    return step_resident_kernel<L, S, COL, FORCE, BLEND>;
+  }
+  template <class F>
+  static cudaError_t with_resident_kernel(const DeviceState &d, F &&f) {
+    auto fb = [&](auto col) {
+      constexpr int COL = decltype(col)::value;
+      if (d.forcing) return d.blend ? f(resident_kernel<COL, true, true>()) : f(resident_kernel<COL, true, false>());
+      return d.blend ? f(resident_kernel<COL, false, true>()) : f(resident_kernel<COL, false, false>());
+    };
+    switch (d.col) {
+      case COL_BGK: return fb(std::integral_constant<int, COL_BGK>{});
+      case COL_BGK_SMAG: return fb(std::integral_constant<int, COL_BGK_SMAG>{});
+      case COL_MRT_NC: return fb(std::integral_constant<int, COL_MRT_NC>{});
+      default: return fb(std::integral_constant<int, COL_MRT>{});
+    }
+  }
+  static cudaLaunchConfig_t resident_config(const DeviceState &d, cudaLaunchAttribute &attr, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)d.resident_cluster);
+    cfg.blockDim = dim3((unsigned)((d.resident_per + 31) / 32 * 32));
+    cfg.dynamicSmemBytes = 2 * (size_t)L::Q * d.resident_per * sizeof(S);
+    cfg.stream = st;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)d.resident_cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+  // Shared memory and cluster size beyond the portable limits, allowed per
+  // kernel (cheap, and the same value every time for a kernel and a size).
+  static cudaError_t allow_resident(const void *kern, const cudaLaunchConfig_t &cfg) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RESIDENT_SMEM);
+    return e;
+  }
+  static cudaError_t resident(const DeviceState &d, long long t, int steps, cudaStream_t st) {
+    if constexpr (L::DIM == 2) {
+      const StepArgs<C> a = make_args(d, t, false, 0, plane_count(d), false), end = make_args(d, t + steps, false, 0,
+                                                                                             plane_count(d), false);
+      ResidentRun run = {d.resident_per, steps, t, {end.s[0], end.s[1], end.s[2]}, end.odd};
+      return with_resident_kernel(d, [&](auto kern) {
+        cudaLaunchAttribute attr = {};
+        const cudaLaunchConfig_t cfg = resident_config(d, attr, st);
+        const cudaError_t e = allow_resident((const void *)kern, cfg);
+        return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kern, a, run) : e;
+      });
+    } else {
+      return cudaErrorNotSupported;
+    }
+  }
+  // Whether one cluster can hold the domain: a node per thread, at least 256
+  // threads a block (fewer, fuller blocks below 4096 nodes), 16 blocks at most.
+  static cudaError_t plan_resident(DeviceState &d) {
+    d.resident_cluster = 0;
+    if constexpr (L::DIM == 2) {
+      if (!d.auto_kernel || d.n > RESIDENT_MAX_CLUSTER * RESIDENT_MAX_THREADS) return cudaSuccess;
+      int c = 1;
+      while (c < RESIDENT_MAX_CLUSTER && 256LL * c < d.n) c *= 2;
+      d.resident_cluster = c;
+      d.resident_per = (int)((d.n + c - 1) / c);
+      return with_resident_kernel(d, [&](auto kern) {
+        cudaLaunchAttribute attr = {};
+        const cudaLaunchConfig_t cfg = resident_config(d, attr, nullptr);
+        int clusters = 0;
+        cudaError_t e = allow_resident((const void *)kern, cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
+        if (e != cudaSuccess || clusters < 1) {  // no room for it: step by step
+          cudaGetLastError();
+          d.resident_cluster = 0;
+        }
+        return cudaSuccess;
+      });
+    }
+    return cudaSuccess;
+  }
+
   // Chooses the kernel and its launch geometry for a handle (called once by
   // lbmc_init after the device state is filled in).
   static cudaError_t plan(DeviceState &d) {
@@ -225,8 +308,8 @@ struct Launchers {
   }
 
   static const LatticeStorageOps *ops() {
-    static const LatticeStorageOps o = {(int)sizeof(C), (int)sizeof(S), &step, &fetch_population,
-                                        &upload_population, &plan};
+    static const LatticeStorageOps o = {(int)sizeof(C), (int)sizeof(S), &step, &resident, &fetch_population,
+                                        &upload_population, &plan, &plan_resident};
     return &o;
   }
 };
