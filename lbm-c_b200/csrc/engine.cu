@@ -909,7 +909,7 @@ static cudaError_t sweep(lbmc_handle *h, int levels) {
       const int first = p.begin(k, s, levels), planes = p.end(k, s, levels) - first;
       if (k > 0 && s > 0) e = cudaStreamWaitEvent(st[k & 1], h->level_done[(k - 1) & 1][s - 1], 0);
       if (e == cudaSuccess)
-        e = h->ops->step(h->ds, h->step + s, false, false, first, planes, s < levels - 1, st[k & 1]);
+        e = h->ops->step(h->ds, h->step + s, false, false, first, planes, true, s < levels - 1, st[k & 1]);
       if (e == cudaSuccess) e = cudaEventRecord(h->level_done[k & 1][s], st[k & 1]);
     }
   cudaError_t ej = cudaEventRecord(h->join, st[1]);
@@ -945,7 +945,7 @@ extern "C" lbmc_status lbmc_iterate(lbmc_handle *h, int nsteps, unsigned flags) 
     const bool last = s == nsteps - 1;
     const bool store = last && (flags & LBMC_STORE_MACROS);
     const bool diag = last && (flags & LBMC_REDUCE_DIAG);
-    CK(h->ops->step(h->ds, h->step, store, diag, 0, plane_count(h->ds), false, h->stream), "step kernel launch");
+    CK(h->ops->step(h->ds, h->step, store, diag, 0, plane_count(h->ds), false, false, h->stream), "step kernel launch");
     h->step++;
     if (diag) {
       const double *records = h->ds.partials;

@@ -62,10 +62,11 @@ struct LatticeStorageOps {
   int ssize;  // bytes of the storage type
   // One time step at step counter t (shift t mod L) of `planes` planes (z in
   // 3-D, y in 2-D) from plane `first` on, wrapping past the last one; the
-  // whole domain with planes = plane_count().  keep: the next step follows
-  // while these planes are in L2.
-  cudaError_t (*step)(const DeviceState &, long long t, bool store, bool diag, int first, int planes, bool keep,
-                      cudaStream_t);
+  // whole domain with planes = plane_count().  swept: other launches of a
+  // sweep run beside it; keep: the next step follows while these planes are
+  // in L2.
+  cudaError_t (*step)(const DeviceState &, long long t, bool store, bool diag, int first, int planes, bool swept,
+                      bool keep, cudaStream_t);
   // `steps` time steps from step counter t on in one launch (resident_cluster
   // > 0 only; no store, no diagnostics).
   cudaError_t (*resident)(const DeviceState &, long long t, int steps, cudaStream_t);

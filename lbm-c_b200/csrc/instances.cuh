@@ -21,7 +21,8 @@ template <class L, class S>
 struct Launchers {
   using C = typename Storage<S>::C;
 
-  static StepArgs<C> make_args(const DeviceState &d, long long t, bool store, int first, int planes, bool keep) {
+  static StepArgs<C> make_args(const DeviceState &d, long long t, bool store, int first, int planes, bool keep,
+                               int block_planes = 1) {
     StepArgs<C> a;
     a.f = d.f;
     a.pitch = d.pitch;
@@ -61,16 +62,40 @@ struct Launchers {
     a.mlp = d.closure_consts;
     // The last blocks, as many as one wave of the chip holds, let the next
     // step come up.
-    const long long per_row = grid_dim(d, planes).x, rows = (long long)planes * (d.dim == 3 ? d.L[1] : 1);
-    const long long wave = (long long)B200_SMS * (d.col == COL_BGK_MLP1   ? direct_min_blocks<S, COL_BGK_MLP1>()
-                                                  : d.col == COL_BGK_MLP ? direct_min_blocks<S, COL_BGK_MLP>()
-                                                  : d.col == COL_BGK_SMAG ? direct_min_blocks<S, COL_BGK_SMAG>()
-                                                                          : direct_min_blocks<S, COL_BGK>());
-    a.release_row = (int)(rows - (wave + per_row - 1) / per_row);
+    const dim3 g = grid_dim(d, (planes + block_planes - 1) / block_planes);
+    a.release_row = (int)((long long)g.y * g.z - (wave(d) + g.x - 1) / g.x);
     a.first_plane = first;
+    a.end_plane = (first + planes - 1) % plane_count(d) + 1;
     a.keep = keep ? 1 : 0;
     a.sr_seed = sr_step_seed(t);
     return a;
+  }
+
+  // Blocks of the direct kernel that the chip holds at a time.
+  static long long wave(const DeviceState &d) {
+    return (long long)B200_SMS * (d.col == COL_BGK_MLP1   ? direct_min_blocks<S, COL_BGK_MLP1>()
+                                  : d.col == COL_BGK_MLP  ? direct_min_blocks<S, COL_BGK_MLP>()
+                                  : d.col == COL_BGK_SMAG ? direct_min_blocks<S, COL_BGK_SMAG>()
+                                                          : direct_min_blocks<S, COL_BGK>());
+  }
+
+  // Whether a block of the direct kernel may take two planes one after the
+  // other: that halves the blocks, whose start-up (dispatch, parameters) costs
+  // the steps that HBM does not hold back.  Tiled AA, us a step with one and
+  // two planes: BF16 Smagorinsky 256^3 236 and 227, FP16 with stochastic rounding
+  // 250 and 245, D2Q9 FP32 4096x2048 102 and 89; FP32 D3Q15 256^3 254 and 258.
+  template <int COL>
+  static constexpr bool two_planes() {
+    return (sizeof(S) == 2 || L::DIM == 2) && !learned_closure(COL);
+  }
+  // ... and where it does: the coarser last wave costs more than the start-up
+  // (64^3 6.5 -> 8.1 us, FP16 192^3 102 -> 105) unless another slab of a sweep
+  // fills it, or in D2Q9 from 16 waves on (2048x2048 FP16 48.3 -> 47.1).
+  static int planes_per_block(const DeviceState &d, int planes, bool swept, bool diag) {
+    const bool can = (sizeof(S) == 2 || L::DIM == 2) && !learned_closure(d.col);
+    if (!can || !d.tiled || diag || planes < 2) return 1;
+    const dim3 g = grid_dim(d, planes);
+    return swept || (L::DIM == 2 && (long long)g.x * g.y * g.z >= 16 * wave(d)) ? 2 : 1;
   }
 
   // One block row per (y, z); blocks of up to STEP_BLOCK threads along x.
@@ -107,7 +132,7 @@ struct Launchers {
   }
 
   template <int COL, bool FORCE, bool BLEND, bool DIAG>
-  static cudaError_t launch(const StepArgs<C> &a, const DeviceState &d, int planes, cudaStream_t st) {
+  static cudaError_t launch(const StepArgs<C> &a, const DeviceState &d, int planes, int block_planes, cudaStream_t st) {
     // The learned closure evaluates its network warp-wide, which the direct
     // kernel's converged warps allow: it never runs in the pipelined kernel.
     if constexpr (!learned_closure(COL)) {
@@ -124,8 +149,14 @@ struct Launchers {
         return cudaSuccess;
       }
     }
-    auto run = [&](auto kern) { return launch_chained(kern, grid_dim(d, planes), block_dim(d), st, a); };
+    auto run = [&](auto kern) {
+      return launch_chained(kern, grid_dim(d, (planes + block_planes - 1) / block_planes), block_dim(d), st, a);
+    };
     if (!d.aa) return run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_SHIFT>);
+    if constexpr (!DIAG && two_planes<COL>())
+      if (block_planes == 2)
+        return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_ODD, 2>)
+                     : run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_EVEN, 2>);
     if (d.tiled)
       return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_ODD>)
                    : run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_EVEN>);
@@ -134,24 +165,27 @@ struct Launchers {
   }
 
   template <int COL, bool BLEND>
-  static cudaError_t launch_fd(const StepArgs<C> &a, const DeviceState &d, bool diag, int planes, cudaStream_t st) {
+  static cudaError_t launch_fd(const StepArgs<C> &a, const DeviceState &d, bool diag, int planes, int block_planes,
+                               cudaStream_t st) {
     if (d.forcing) {
-      if (diag) return launch<COL, true, BLEND, true>(a, d, planes, st);
-      return launch<COL, true, BLEND, false>(a, d, planes, st);
+      if (diag) return launch<COL, true, BLEND, true>(a, d, planes, block_planes, st);
+      return launch<COL, true, BLEND, false>(a, d, planes, block_planes, st);
     }
-    if (diag) return launch<COL, false, BLEND, true>(a, d, planes, st);
-    return launch<COL, false, BLEND, false>(a, d, planes, st);
+    if (diag) return launch<COL, false, BLEND, true>(a, d, planes, block_planes, st);
+    return launch<COL, false, BLEND, false>(a, d, planes, block_planes, st);
   }
 
   template <int COL>
-  static cudaError_t launch_col(const StepArgs<C> &a, const DeviceState &d, bool diag, int planes, cudaStream_t st) {
-    if (d.blend) return launch_fd<COL, true>(a, d, diag, planes, st);
-    return launch_fd<COL, false>(a, d, diag, planes, st);
+  static cudaError_t launch_col(const StepArgs<C> &a, const DeviceState &d, bool diag, int planes, int block_planes,
+                               cudaStream_t st) {
+    if (d.blend) return launch_fd<COL, true>(a, d, diag, planes, block_planes, st);
+    return launch_fd<COL, false>(a, d, diag, planes, block_planes, st);
   }
 
-  static cudaError_t step(const DeviceState &d, long long t, bool store, bool diag, int first, int planes, bool keep,
-                          cudaStream_t st) {
-    const StepArgs<C> a = make_args(d, t, store, first, planes, keep);
+  static cudaError_t step(const DeviceState &d, long long t, bool store, bool diag, int first, int planes, bool swept,
+                          bool keep, cudaStream_t st) {
+    const int block_planes = planes_per_block(d, planes, swept, diag);
+    const StepArgs<C> a = make_args(d, t, store, first, planes, keep, block_planes);
     if (d.n_sf > 0) {
       const int nb = (d.n_sf + 127) / 128;
       sf_gather_kernel<L, S><<<nb, 128, 0, st>>>(a, d.sf_nodes, d.sf_face, d.n_sf,
@@ -159,12 +193,12 @@ struct Launchers {
     }
     cudaError_t e;
     switch (d.col) {
-      case COL_BGK: e = launch_col<COL_BGK>(a, d, diag, planes, st); break;
-      case COL_BGK_SMAG: e = launch_col<COL_BGK_SMAG>(a, d, diag, planes, st); break;
-      case COL_MRT_NC: e = launch_col<COL_MRT_NC>(a, d, diag, planes, st); break;
-      case COL_BGK_MLP: e = launch_col<COL_BGK_MLP>(a, d, diag, planes, st); break;
-      case COL_BGK_MLP1: e = launch_col<COL_BGK_MLP1>(a, d, diag, planes, st); break;
-      default: e = launch_col<COL_MRT>(a, d, diag, planes, st); break;
+      case COL_BGK: e = launch_col<COL_BGK>(a, d, diag, planes, block_planes, st); break;
+      case COL_BGK_SMAG: e = launch_col<COL_BGK_SMAG>(a, d, diag, planes, block_planes, st); break;
+      case COL_MRT_NC: e = launch_col<COL_MRT_NC>(a, d, diag, planes, block_planes, st); break;
+      case COL_BGK_MLP: e = launch_col<COL_BGK_MLP>(a, d, diag, planes, block_planes, st); break;
+      case COL_BGK_MLP1: e = launch_col<COL_BGK_MLP1>(a, d, diag, planes, block_planes, st); break;
+      default: e = launch_col<COL_MRT>(a, d, diag, planes, block_planes, st); break;
     }
     if (e != cudaSuccess) return e;
     return cudaGetLastError();

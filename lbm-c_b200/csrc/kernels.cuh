@@ -367,6 +367,7 @@ struct StepArgs {
   const MlpStep *closure;       // learned closure (COL_BGK_MLP, COL_BGK_MLP1): weights
   MlpConsts mlp;                // and its scalars
   int first_plane;              // direct kernel: plane of block row 0 (z in 3-D, y in 2-D)
+  int end_plane;                // PLANES > 1: the plane (not wrapped) after the launch's last one, 1 .. L
   int keep;                     // direct kernel: the next step follows while the planes are in L2
   int release_row;              // direct kernel: block rows from here on release the next step
   unsigned sr_seed;             // stochastic-rounding seed of this step (sr_step_seed(t))
@@ -1288,7 +1289,10 @@ constexpr int direct_min_blocks() {
   return COL == COL_BGK_SMAG ? DIRECT_MIN_BLOCKS_SMAG : DIRECT_MIN_BLOCKS;
 }
 
-template <class L, class S, int COL, bool FORCE, bool BLEND, bool DIAG, int STREAM>
+// PLANES: planes that a block takes one after the other (no DIAG, whose
+// partials go by block row).  As a run-time count the loop cost the one-plane
+// launches 3-10% (FP32 256^3 255 -> 263 us).
+template <class L, class S, int COL, bool FORCE, bool BLEND, bool DIAG, int STREAM, int PLANES = 1>
 __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
     step_kernel(const StepArgs<typename Storage<S>::C> a) {
   using C = typename Storage<S>::C;
@@ -1298,8 +1302,8 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   // The grid covers whole planes from first_plane on, past the last one from
   // plane 0 again.
   int cy = blockIdx.y, cz = blockIdx.z;
-  if constexpr (L::DIM == 3) cz = wrap_add(cz, a.first_plane, a.L[2]);
-  else cy = wrap_add(cy, a.first_plane, a.L[1]);
+  if constexpr (L::DIM == 3) cz = wrap_add(cz * PLANES, a.first_plane, a.L[2]);
+  else cy = wrap_add(cy * PLANES, a.first_plane, a.L[1]);
   // Read slot of population i: (i, slot(i)) in the shift layout, (i, n) at
   // an AA-even step, (opp(i), slot(i)) with the t = 1 shift at an AA-odd
   // step; out[i] goes back to slot(i) (shift) or to population opp(i)'s
@@ -1335,6 +1339,14 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   if constexpr (!learned_closure(COL)) {
     if (!DIAG && !active) return;
     if (active) {
+      wait_for_predecessor();
+#pragma unroll 1
+      for (int part = 0; part < PLANES; part++) {
+      if (part > 0) {  // the block's next plane, unless the launch ends before it
+        int &plane = L::DIM == 3 ? cz : cy;
+        if (plane + 1 == a.end_plane) break;
+        plane = wrap_add(plane, 1, a.L[L::DIM - 1]);
+      }
       const C inv_scale = a.inv_scale, scale = a.scale;
       Sites st;
       TiledSites ts;
@@ -1342,7 +1354,6 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       const int n = x + a.L[0] * (cy + a.L[1] * cz);
       S *f = reinterpret_cast<S *>(a.f);
       Node<L, C> nd;
-      wait_for_predecessor();
       unroll<Q>([&](auto ic) { nd.g[decltype(ic)::value] = load_dev(read_at(f, st, ts, n, ic), inv_scale); });
       const int cls = a.cls[n];
       C out[Q];
@@ -1381,6 +1392,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
         store_all(st, ts);
       }
       store_and_reduce(nd, a, n, dv, nonfinite, DIAG);
+      }
     }
   } else {
     // The learned closure's network runs warp-wide: every lane of a warp

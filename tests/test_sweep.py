@@ -30,6 +30,10 @@ def test_order_of_a_sweep(tmp_path):
     ("d3q15", (215, 205, 203), "f16sr", "shift", dict(collision_type=0, forcing=True)),
     ("d2q9", (2311, 2011, 1), "f32", "aa", dict(collision_type=1, forcing=True, solids=0.2, partial=0.2)),
     ("d2q9", (1601, 1503, 1), "f64", "shift", dict(collision_type=0, macro="random")),
+    # two planes a block: odd planes, a slab and a launch that end on half a block
+    ("d3q15", (256, 193, 181), "bf16", "aa", dict(collision_type=2, micro="zh", solids=0.2)),
+    ("d3q15", (192, 219, 217), "f16", "aa", dict(collision_type=0, c_smag=0.1)),
+    ("d2q9", (2304, 2051, 1), "f32", "aa", dict(collision_type=1, forcing=True, partial=0.2)),
 ])
 def test_sweep_equals_single_steps(lbmc, lattice, length, storage, streaming, kw):
     case = make_case(lattice, length, seed=4, **kw)
