@@ -22,7 +22,7 @@ struct Launchers {
   using C = typename Storage<S>::C;
 
   static StepArgs<C> make_args(const DeviceState &d, long long t, bool store, int first, int planes, bool keep,
-                               int block_planes = 1) {
+                               int block_planes = 1, bool flat = false) {
     StepArgs<C> a;
     a.f = d.f;
     a.pitch = d.pitch;
@@ -62,8 +62,15 @@ struct Launchers {
     a.mlp = d.closure_consts;
     // The last blocks, as many as one wave of the chip holds, let the next
     // step come up.
-    const dim3 g = grid_dim(d, (planes + block_planes - 1) / block_planes);
-    a.release_row = (int)((long long)g.y * g.z - (wave(d) + g.x - 1) / g.x);
+    const long long plane_nodes = d.n / plane_count(d);
+    a.first_node = (int)(first * plane_nodes);
+    a.span = (int)(planes * plane_nodes);
+    if (flat) {
+      a.release_row = (int)(((long long)a.span + DIRECT_BLOCK - 1) / DIRECT_BLOCK - wave(d));
+    } else {
+      const dim3 g = grid_dim(d, (planes + block_planes - 1) / block_planes);
+      a.release_row = (int)((long long)g.y * g.z - (wave(d) + g.x - 1) / g.x);
+    }
     a.first_plane = first;
     a.end_plane = (first + planes - 1) % plane_count(d) + 1;
     a.keep = keep ? 1 : 0;
@@ -160,8 +167,11 @@ struct Launchers {
     if (d.tiled)
       return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_ODD>)
                    : run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AAT_EVEN>);
-    return a.odd ? run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_ODD>)
-                 : run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_EVEN>);
+    if (a.odd) return run(step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_ODD>);
+    auto even = step_kernel<L, S, COL, FORCE, BLEND, DIAG, STREAM_AA_EVEN>;
+    if constexpr (flat_step<COL, DIAG, STREAM_AA_EVEN>())
+      return launch_chained(even, dim3((unsigned)((a.span + DIRECT_BLOCK - 1) / DIRECT_BLOCK)), dim3(DIRECT_BLOCK), st, a);
+    return run(even);
   }
 
   template <int COL, bool BLEND>
@@ -185,7 +195,8 @@ struct Launchers {
   static cudaError_t step(const DeviceState &d, long long t, bool store, bool diag, int first, int planes, bool swept,
                           bool keep, cudaStream_t st) {
     const int block_planes = planes_per_block(d, planes, swept, diag);
-    const StepArgs<C> a = make_args(d, t, store, first, planes, keep, block_planes);
+    const bool flat = d.aa && !d.tiled && !(t & 1) && !diag && !learned_closure(d.col);  // flat_step()
+    const StepArgs<C> a = make_args(d, t, store, first, planes, keep, block_planes, flat);
     if (d.n_sf > 0) {
       const int nb = (d.n_sf + 127) / 128;
       sf_gather_kernel<L, S><<<nb, 128, 0, st>>>(a, d.sf_nodes, d.sf_face, d.n_sf,

@@ -367,6 +367,7 @@ struct StepArgs {
   const MlpStep *closure;       // learned closure (COL_BGK_MLP, COL_BGK_MLP1): weights
   MlpConsts mlp;                // and its scalars
   int first_plane;              // direct kernel: plane of block row 0 (z in 3-D, y in 2-D)
+  int first_node, span;         // flat step: first node, nodes of the launch
   int end_plane;                // PLANES > 1: the plane (not wrapped) after the launch's last one, 1 .. L
   int keep;                     // direct kernel: the next step follows while the planes are in L2
   int release_row;              // direct kernel: block rows from here on release the next step
@@ -1289,6 +1290,15 @@ constexpr int direct_min_blocks() {
   return COL == COL_BGK_SMAG ? DIRECT_MIN_BLOCKS_SMAG : DIRECT_MIN_BLOCKS;
 }
 
+// The plain AA layout's even step touches only a node's own slots: it runs
+// over the node index, so that only its last warp has idle lanes whatever Lx
+// is (us a step, FP32 150x143x161 79.0 -> 71.5, Smagorinsky BF16 70^3 11.5
+// -> 9.4, FP64 150^3 119 -> 112).  Diagnostic partials go by block row.
+template <int COL, bool DIAG, int STREAM>
+__host__ __device__ constexpr bool flat_step() {
+  return STREAM == STREAM_AA_EVEN && !DIAG && !learned_closure(COL);
+}
+
 // PLANES: planes that a block takes one after the other (no DIAG, whose
 // partials go by block row).  As a run-time count the loop cost the one-plane
 // launches 3-10% (FP32 256^3 255 -> 263 us).
@@ -1297,8 +1307,10 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
     step_kernel(const StepArgs<typename Storage<S>::C> a) {
   using C = typename Storage<S>::C;
   constexpr int Q = L::Q;
+  // FLAT: the step needs no coordinates, blocks take 64 consecutive nodes.
+  constexpr bool FLAT = flat_step<COL, DIAG, STREAM>();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = x < a.L[0];
+  const bool active = x < (FLAT ? a.span : a.L[0]);
   // The grid covers whole planes from first_plane on, past the last one from
   // plane 0 again.
   int cy = blockIdx.y, cz = blockIdx.z;
@@ -1335,7 +1347,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   // block counts as having done so): released from every block, the FP16
   // 192^3 step took 115 instead of 103 us.  The class byte is read after the
   // wait; before it, the learned closure's step was 5% slower.
-  if ((int)(blockIdx.y + gridDim.y * blockIdx.z) >= a.release_row) release_successor();
+  if ((int)(FLAT ? blockIdx.x : blockIdx.y + gridDim.y * blockIdx.z) >= a.release_row) release_successor();
   if constexpr (!learned_closure(COL)) {
     if (!DIAG && !active) return;
     if (active) {
@@ -1351,7 +1363,13 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       Sites st;
       TiledSites ts;
       init_sites(st, ts);
-      const int n = x + a.L[0] * (cy + a.L[1] * cz);
+      int n;
+      if constexpr (FLAT) {
+        const unsigned m = (unsigned)a.first_node + (unsigned)x;
+        n = (int)(m >= (unsigned)a.n ? m - (unsigned)a.n : m);
+      } else {
+        n = x + a.L[0] * (cy + a.L[1] * cz);
+      }
       S *f = reinterpret_cast<S *>(a.f);
       Node<L, C> nd;
       unroll<Q>([&](auto ic) { nd.g[decltype(ic)::value] = load_dev(read_at(f, st, ts, n, ic), inv_scale); });
