@@ -419,8 +419,8 @@ def run_batch(args, world, rank, local):
 
 def reference_built() -> bool:
     """Whether the host-compiled reference step (oracle/build_ref.sh) is here."""
-    from oracle.oracle import REF_DIR
-    return os.path.exists(os.path.join(REF_DIR, "libref_d3q15_patched.so"))
+    from oracle.oracle import reference_available
+    return reference_available("d3q15", "patched")
 
 
 class ReferenceTimer:
