@@ -816,17 +816,22 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
       } else {
         // f_eq(rho, u) of collision.cu:58.
         const double w = lattice_w(d.lattice, i);
-        parallel_for(n, [&](long long b, long long e, int) {
+        const int dim = d.dim;
+        const double *const rho_in = dom->rho, *const u_in[3] = {dom->u[0], dom->u[1], dom->u[2]};
+        double ei[3] = {0, 0, 0};
+        for (int c = 0; c < dim; c++) ei[c] = lattice_e(d.lattice, c, i);
+        double *const out_f = host.data();
+        parallel_for(n, [=](long long b, long long e, int) {
           for (long long k = b; k < e; k++) {
-            const double rho = dom->rho ? dom->rho[k] : 1.0;
-            double u[3] = {0, 0, 0}, usq = 0, eu = 0;
-            for (int c = 0; c < d.dim; c++) {
-              u[c] = dom->u[c] ? dom->u[c][k] : 0.0;
-              usq += u[c] * u[c];
-              eu += lattice_e(d.lattice, c, i) * u[c];
+            const double rho = rho_in ? rho_in[k] : 1.0;
+            double usq = 0, eu = 0;
+            for (int c = 0; c < dim; c++) {
+              const double u = u_in[c] ? u_in[c][k] : 0.0;
+              usq += u * u;
+              eu += ei[c] * u;
             }
             eu *= 3.0;
-            host[k] = rho * w * (1.0 + eu + 0.5 * eu * eu - 1.5 * usq);
+            out_f[k] = rho * w * (1.0 + eu + 0.5 * eu * eu - 1.5 * usq);
           }
         });
       }
