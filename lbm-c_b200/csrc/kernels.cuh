@@ -1347,7 +1347,15 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
   // block counts as having done so): released from every block, the FP16
   // 192^3 step took 115 instead of 103 us.  The class byte is read after the
   // wait; before it, the learned closure's step was 5% slower.
-  if ((int)(FLAT ? blockIdx.x : blockIdx.y + gridDim.y * blockIdx.z) >= a.release_row) release_successor();
+  // The learned closure releases after the network instead: blocks that come
+  // up while this step's still compute settle unevenly over the SMs, and the
+  // passes are bound by an SM's own rate and latency (us a step with plain
+  // launches, released at the start, after the network: 32^3 8 passes 12.8,
+  // 17.3, 9.4; 24^3 10.1, 12.4, 7.0; 64^3 2 passes 21.0, 17.9, 17.7).
+  auto release = [&]() {
+    if ((int)(FLAT ? blockIdx.x : blockIdx.y + gridDim.y * blockIdx.z) >= a.release_row) release_successor();
+  };
+  if constexpr (!learned_closure(COL)) release();
   if constexpr (!learned_closure(COL)) {
     if (!DIAG && !active) return;
     if (active) {
@@ -1444,6 +1452,7 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
         nd.u[0] = nd.u[1] = nd.u[2] = 0;
       }
       collide_fluid<L, C, COL, FORCE, BLEND>(nd, a, n, fluid && cls ? a.table[cls] : 0u, out, fluid);
+      release();
       if (!fluid) collide_solid(nd, out);
       if (active) {
         // The store sites equal the load sites; recomputing them is cheaper
