@@ -1141,8 +1141,12 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
         __shared__ __align__(16) unsigned mlp_stage[DIRECT_BLOCK / 32][128];
         // The node's state waits in shared memory meanwhile (one column per
         // thread, no conflicts): held in registers beside the network it
-        // took 128 of them, 8 blocks per SM (DIRECT_MIN_BLOCKS_MLP1).
-        __shared__ C node_state[L::Q + 13][DIRECT_BLOCK];
+        // took 128 of them, 8 blocks per SM (DIRECT_MIN_BLOCKS_MLP1).  FP64
+        // has 8 blocks either way: its single pass keeps the registers (128^3
+        // 111.4 -> 108.5 us a step), its pass loop gains from the column
+        // (two passes 150 -> 141).
+        constexpr bool PARK = sizeof(C) == 4 || COL == COL_BGK_MLP;
+        __shared__ C node_state[PARK ? L::Q + 13 : 1][DIRECT_BLOCK];
         auto each_state = [&](auto &&f) {
           unroll<L::Q>([&](auto ic) { f(nd.g[decltype(ic)::value], decltype(ic)::value); });
           unroll<3>([&](auto dc) {
@@ -1154,10 +1158,17 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
           });
           f(nd.drho, L::Q + 6);
         };
-        each_state([&](C &v, int k) { *(volatile C *)&node_state[k][threadIdx.x] = v; });
-        unroll<6>([&](auto cc) {
-          *(volatile C *)&node_state[L::Q + 7 + decltype(cc)::value][threadIdx.x] = q[decltype(cc)::value];
-        });
+        if constexpr (PARK) {
+          each_state([&](C &v, int k) { *(volatile C *)&node_state[k][threadIdx.x] = v; });
+          unroll<6>([&](auto cc) {
+            *(volatile C *)&node_state[L::Q + 7 + decltype(cc)::value][threadIdx.x] = q[decltype(cc)::value];
+          });
+        }
+        auto q_at = [&](auto cc) -> C {
+          constexpr int c = decltype(cc)::value;
+          if constexpr (PARK) return *(volatile C *)&node_state[L::Q + 7 + c][threadIdx.x];
+          else return q[c];
+        };
         const MlpStep *cl = a.closure;
         bool in_range = participate;
         C tau_l = tau_smag;
@@ -1167,8 +1178,7 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
         for (int it = 0; it < passes; it++) {
           const float ks = __fdividef(-1.5f, (float)(nd.rho * tau_l));
           float Sm[6], f[MLP_IN];
-#pragma unroll
-          for (int c = 0; c < 6; c++) Sm[c] = ks * (float)*(volatile C *)&node_state[L::Q + 7 + c][threadIdx.x];
+          unroll<6>([&](auto cc) { Sm[decltype(cc)::value] = ks * (float)q_at(cc); });
           strain_features(Sm, (float)nd.rho, f);
 #pragma unroll
           for (int c = 0; c < MLP_IN; c++) {
@@ -1181,7 +1191,7 @@ __device__ __forceinline__ void collide_fluid(Node<L, C> &nd, const StepArgs<C> 
           if (in_range) tau_l = tau0 + C(3) * C(fmaxf(0.0f, a.mlp.target_scale * y));
         }
         tau = in_range ? tau_l : tau_smag;
-        each_state([&](C &v, int k) { v = *(volatile C *)&node_state[k][threadIdx.x]; });
+        if constexpr (PARK) each_state([&](C &v, int k) { v = *(volatile C *)&node_state[k][threadIdx.x]; });
       }
     }
     // 1/tau: the host's value for a uniform tau, else the local one
