@@ -78,7 +78,8 @@ def profiled_traffic(kernel_tag: str):
 
 def step_launches(w, storage: str, kernel: str, closure: bool, steps: int) -> int:
     """Step-kernel launches of one lbmc_iterate(steps) without flags: the
-    grouping of csrc/sweep.h and of the small 2-D domains, restated."""
+    grouping of csrc/sweep.h and of the small 2-D domains, restated (without
+    sweep.h's limit on long rows of 2-D domains, which no workload here has)."""
     if closure or kernel == "pipelined":
         return steps
     if w.dim == 2 and w.n <= 16384 and kernel == "auto" and steps >= 6:

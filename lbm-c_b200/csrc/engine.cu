@@ -815,7 +815,9 @@ extern "C" lbmc_status lbmc_init(const lbmc_config *cfg, const lbmc_domain *dom,
 
   // Stress-free nodes need a pre-pass over the whole domain before each step,
   // and the bulk-copy kernel walks all rows: both go step by step.
-  if (d.n_sf == 0 && !d.use_pipeline) h->sweep = plan_sweep(plane_count(d), n / plane_count(d) * q * ss, ss);
+  if (d.n_sf == 0 && !d.use_pipeline)
+    h->sweep = plan_sweep(plane_count(d), n / plane_count(d) * q * ss, ss,
+                          sweep_plane_limit(d.dim, ss, d.tiled, d.col == COL_BGK_SMAG, d.blend, d.forcing));
   if (h->sweep.depth > 1) TRYCUDA(make_sweep(h), "sweep streams");
   if (d.n_sf == 0 && !d.use_pipeline) TRYCUDA(h->ops->plan_resident(d), "kernel planning");
 

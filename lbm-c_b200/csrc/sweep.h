@@ -18,6 +18,7 @@
 #pragma once
 
 #include <algorithm>
+#include <climits>
 
 namespace lbmc {
 
@@ -57,10 +58,12 @@ struct SweepPlan {
 //     not, FP64 128^3 (252 MB) 68 and 92.  2-byte storage, bound by
 //     instruction issue before HBM, starts to gain later: FP16 192^3 (212 MB)
 //     104.4 and 103.5, 256^3 (503 MB) 250 and 262; its line is 2 x L2.
-inline SweepPlan plan_sweep(int planes, long long plane_bytes, int elem) {
+//   - Planes above plane_limit bytes (sweep_plane_limit): step by step.
+inline SweepPlan plan_sweep(int planes, long long plane_bytes, int elem, long long plane_limit = LLONG_MAX) {
   constexpr long long L2 = 126ll << 20, SLAB = 30ll << 20, WINDOW = 96ll << 20;
   SweepPlan p;
   p.planes = planes;
+  if (plane_bytes > plane_limit) return p;
   if (plane_bytes * planes <= (elem > 2 ? L2 + L2 / 4 : 2 * L2)) return p;
   p.slab = (int)std::max(1ll, SLAB / plane_bytes);
   const long long skew = WINDOW / plane_bytes - 2 * p.slab;
@@ -68,6 +71,33 @@ inline SweepPlan plan_sweep(int planes, long long plane_bytes, int elem) {
   const long long room = (planes - 2 * p.slab - 1) / 2;
   p.depth = (int)std::max(1ll, std::min<long long>(SweepPlan::MAX_DEPTH, std::min(skew, room)));
   return p;
+}
+
+// The largest plane of a domain that gains from sweeps.  3-D domains gain, or
+// lose 1% at most (2-byte storage in the shift layout), up to the planes that
+// leave no second level.  In 2-D a plane is a row, one step of a short slab of
+// long rows is a launch of few blocks, and the step of 2-byte storage is near
+// its issue limit without a sweep.  us a step of ~20 M nodes, step by step ->
+// swept, by row length:
+//   - FP64: 300000 tiled 456 -> 411; never slower.
+//   - FP32, tiled AA or partly solid nodes: 64000 230 -> 173, 300000 233 ->
+//     211, 600000 (21.6 MB) 232 -> 328; partly solid in the shift layout
+//     300000 338 -> 318, 600000 337 -> 345.  Line: 12 MB.
+//   - FP32 otherwise: 100000 (3.6 MB) 267 -> 261, 120000 259 -> 259, 150000
+//     (5.4 MB) 266 -> 279, 600000 262 -> 321.  Line: 4 MB.
+//   - 2-byte storage, tiled AA: FP16 64000 175 -> 163, 150000 (2.7 MB) 173 ->
+//     176, 200000 173 -> 163, 300000 (5.4 MB) 174 -> 192.  Line: 4 MB.
+//   - 2-byte storage otherwise: FP16 BGK 6000 199 -> 215, 150000 198 -> 229, MRT
+//     4000 161 -> 170, forced BGK 100000 209 -> 212: none.  With Smagorinsky or
+//     with partly solid nodes and a force, whose steps are longer: 4000 189 ->
+//     184 and 216 -> 207, 100000 (1.8 MB) 204 -> 200 and 235 -> 227, 150000
+//     (2.7 MB) 248 -> 257 and 281 -> 281.  Line: 2 MB.
+inline long long sweep_plane_limit(int dim, int elem, bool tiled, bool smagorinsky, bool partly_solid, bool forcing) {
+  constexpr long long MB = 1ll << 20;
+  if (dim == 3 || elem == 8) return LLONG_MAX;
+  if (elem == 4) return tiled || partly_solid ? 12 * MB : 4 * MB;
+  if (tiled) return 4 * MB;
+  return smagorinsky || (partly_solid && forcing) ? 2 * MB : 0;
 }
 
 }  // namespace lbmc
