@@ -269,9 +269,9 @@ typedef struct lbmc_batch_config {
   int wide_min_nodes;   /* domains too large for shared memory with at least this many nodes
                            are stepped one step per launch over every SM, the others one block
                            per domain, K steps per launch; 0 = default: 3/4 of an SM's share
-                           of all nodes, at least 2048 and with FP32 at most 32768, and
-                           domains above the share go wide even if they would fit in
-                           shared memory */
+                           of all nodes, at least 2048 and with FP32 at most 32768, and the
+                           largest of the domains that fit in shared memory go wide as far
+                           as that shortens the estimated step */
   int wide_below;       /* the one-block-per-domain ones join the wide path once fewer than
                            this many of them are running; 0 = default (half the SMs), < 0 =
                            never */

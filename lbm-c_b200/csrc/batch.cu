@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "../../include/lbmc.h"
+#include "batch_split.h"
 #include "engine_internal.h"
 #include "kernels.cuh"
 #include "launch.cuh"
@@ -56,7 +57,7 @@ struct BatchDomainDev {
   long long node_off;  // offset into class / porosity / u_prev arrays
   int pitch;           // elements between populations (global)
   int lx, ly;
-  int resident;        // fits in shared memory
+  int resident;        // stepped in shared memory
 };
 
 struct BatchStateDev {
@@ -722,25 +723,42 @@ extern "C" lbmc_status lbmc_batch_init(const lbmc_batch_config *cfg, int ndomain
     }
   }
   // Which domains one SM steps by itself (shared memory, or one block in HBM)
-  // and which go over every SM.  One SM's domain must not outlast the launch:
-  // it is kept to 3/4 of an SM's share of all nodes, with a floor of 2048
-  // nodes, whose step takes a block about as long (3 us) as the shortest wide
-  // launch.  Measured, GLUPS without -> with the line: 192 domains FP16 15.6
-  // -> 65, 24 FP16 40 -> 53, 40 BF16 48 -> 63; at 3/2 of the share 192 FP16
-  // ran 49.  FP32 domains also go wide from 32768 nodes up: the 4096-domain
-  // sweep ran 52.3 / 55.4 / 54.1 / 52.0 / 50.3 GLUPS for thresholds 1 / 32768 /
-  // 65536 / 131072 / none, FP16 66.1 / 71.2 / 74.7 / 78.2 / 80.2 (2-byte domains
-  // stepped K times by one block stay in cache).
+  // and which go over every SM.  Of those that fit in shared memory,
+  // batch_split.h chooses.  An HBM domain must not outlast the launch: one
+  // block steps those of up to 3/4 of an SM's share of all nodes, with a floor
+  // of 2048 nodes, whose step takes a block about as long (3 us) as the
+  // shortest wide launch.  Measured, GLUPS without -> with the line: 192
+  // domains FP16 15.6 -> 65, 24 FP16 40 -> 53, 40 BF16 48 -> 63; at 3/2 of the
+  // share 192 FP16 ran 49.  FP32 domains also go wide from 32768 nodes up: the
+  // 4096-domain sweep ran 52.3 / 55.4 / 54.1 / 52.0 / 50.3 GLUPS for thresholds
+  // 1 / 32768 / 65536 / 131072 / none, FP16 66.1 / 71.2 / 74.7 / 78.2 / 80.2
+  // (2-byte domains stepped K times by one block stay in cache).  (296 FP32
+  // domains of 100x100, two to an SM: 44 us a step, wide 55.)
   const long long share = std::max(2048LL, 3 * b->total_nodes / (4 * b->sms));
+  auto nodes = [&](int d) { return (long long)b->dom[d].lx * b->dom[d].ly; };
+  std::vector<char> goes_wide(ndomains, 0);  // though it would fit in shared memory
   b->wide_min_nodes = cfg->wide_min_nodes;
   if (b->wide_min_nodes <= 0) {
     b->wide_min_nodes = cfg->storage == LBMC_F32 ? std::min(32768LL, share) : share;
-    for (BatchDomainDev &D : b->dom) D.resident = D.resident && (long long)D.lx * D.ly <= share;
+    std::vector<int> fitting;
+    for (int d = 0; d < ndomains; d++)
+      if (b->dom[d].resident) fitting.push_back(d);
+    std::stable_sort(fitting.begin(), fitting.end(), [&](int x, int y) { return nodes(x) > nodes(y); });
+    std::vector<long long> fit;
+    long long rest = b->total_nodes;
+    for (int d : fitting) {
+      fit.push_back(nodes(d));
+      rest -= nodes(d);
+    }
+    const size_t go = wide_of_fitting(fit, rest, share, b->sms);
+    for (size_t k = 0; k < go; k++) {
+      goes_wide[fitting[k]] = 1;
+      b->dom[fitting[k]].resident = 0;
+    }
   }
   auto klass = [&](int d) {
-    const BatchDomainDev &D = b->dom[d];
-    if (D.resident) return 0;
-    return (long long)D.lx * D.ly >= b->wide_min_nodes ? 2 : 1;
+    if (b->dom[d].resident) return 0;
+    return goes_wide[d] || nodes(d) >= b->wide_min_nodes ? 2 : 1;
   };
   b->order.resize(ndomains);
   std::iota(b->order.begin(), b->order.end(), 0);
