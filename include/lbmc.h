@@ -265,7 +265,8 @@ typedef struct lbmc_batch_config {
   double storage_scale; /* 0 = default (1024 for FP16); FP16: a power of two in [2^-15, 2^14] */
   int device;
   int block_threads;    /* 0 = autotune (256/512/1024) */
-  int steps_per_launch; /* 0 = autotune (check_every or 4*check_every) */
+  int steps_per_launch; /* 0 = autotune (check_every, twice that where it is odd, or
+                           4*check_every) */
   int wide_min_nodes;   /* domains too large for shared memory with at least this many nodes
                            are stepped one step per launch over every SM, the others one block
                            per domain, K steps per launch; 0 = default: 3/4 of an SM's share

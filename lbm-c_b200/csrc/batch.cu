@@ -23,8 +23,8 @@
 // One CUDA graph launch holds the shared-memory kernel, the block-stepped
 // kernel and the K wide steps in three branches.  Every running domain has
 // taken the same number of steps (a domain that stopped is frozen for good),
-// so the host knows each launch's step counter.  Every C steps a domain compares u with its value C steps earlier (max norm) and
-// freezes once below the tolerance, recording the device timer.  The host
+// so the host knows each launch's step counter.  Every C steps a domain
+// compares u with its value C steps earlier (max norm) and freezes once below the tolerance, recording the device timer.  The host
 // replays the graph until every domain converged, stopped or hit the step
 // cap.  Once fewer than wide_below block-stepped domains run, they join the
 // wide path; whenever a quarter of the listed wide domains have stopped,
@@ -38,6 +38,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -471,9 +472,9 @@ struct lbmc_batch {
   int sms = 0;
   int threads = 0, steps = 0;  // tuned launch shape
   int hbm_blocks_per_sm[3] = {1, 1, 1};  // for 256 / 512 / 1024 threads
-  cudaStream_t side = nullptr, blocks = nullptr;  // graph branches of the wide steps, the block-stepped domains
-  cudaEvent_t fork = nullptr, join = nullptr, join_blocks = nullptr;
-  long long t = 0;                        // steps that every running domain has taken
+  cudaStream_t side[2] = {};  // branches of a launch group beside the first
+  cudaEvent_t fork = nullptr, join[2] = {};
+  long long t = 0;            // steps that every running domain has taken
   double scale = 1;
 };
 
@@ -559,27 +560,32 @@ struct WideWork {
   }
 };
 
-// One graph launch from step counter t on, in three branches: the resident
-// kernel on st, the block-stepped kernel (unless its domains moved to the wide
-// path) and the wide steps on streams of their own; joined again.
+// One launch group from step counter t on, in a branch for each class that
+// has work: the resident kernel, the block-stepped kernel (unless its domains
+// moved to the wide path) and the wide steps.  The first takes st, the others
+// fork to streams of their own and join again.
 template <class S>
 cudaError_t launch_round(lbmc_batch *b, const BatchArgs &res, const BatchArgs &blk, const BatchArgs &wid, long long t,
                          int threads, bool run_block, const WideWork &w, cudaStream_t st) {
-  cudaError_t e = cudaEventRecord(b->fork, st);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(b->side, b->fork, 0);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(b->blocks, b->fork, 0);
+  const bool has_res = res.ndomains > 0, has_blk = run_block && blk.ndomains > 0, has_wide = w.nwide > 0;
+  const int forks = std::max(0, has_res + has_blk + has_wide - 1);
+  cudaError_t e = forks > 0 ? cudaEventRecord(b->fork, st) : cudaSuccess;
+  for (int k = 0; k < forks && e == cudaSuccess; k++) e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
   if (e != cudaSuccess) return e;
-  if (res.ndomains > 0) {
+  int taken = 0;
+  auto branch = [&]() { return taken++ == 0 ? st : b->side[taken - 2]; };
+  if (has_res) {
     auto kr = b->blend ? batch_kernel<S, true, true> : batch_kernel<S, false, true>;
-    kr<<<b->sms, threads, b->smem_bytes, st>>>(res);
+    kr<<<b->sms, threads, b->smem_bytes, branch()>>>(res);
   }
-  if (run_block && blk.ndomains > 0) {
+  if (has_blk) {
     const int k = threads <= 256 ? 0 : (threads <= 512 ? 1 : 2);
     auto kh = b->blend ? batch_kernel<S, true, false> : batch_kernel<S, false, false>;
-    kh<<<std::min(blk.ndomains, b->sms * b->hbm_blocks_per_sm[k]), threads, 0, b->blocks>>>(blk);
+    kh<<<std::min(blk.ndomains, b->sms * b->hbm_blocks_per_sm[k]), threads, 0, branch()>>>(blk);
   }
   e = cudaGetLastError();
-  if (w.nwide > 0) {
+  if (has_wide) {
+    const cudaStream_t sw = branch();
     auto even = b->blend ? batch_wide_kernel<S, true, false> : batch_wide_kernel<S, false, false>;
     auto odd = b->blend ? batch_wide_kernel<S, true, true> : batch_wide_kernel<S, false, true>;
     const int grid = (w.nsegs + WIDE_WARPS - 1) / WIDE_WARPS;
@@ -588,21 +594,22 @@ cudaError_t launch_round(lbmc_batch *b, const BatchArgs &res, const BatchArgs &b
       const long long ts = t + s;
       const bool save = ts % wid.check == 0, test = save && ts >= wid.check, last = s == wid.steps - 1;
       // only the last wave of blocks releases the next launch (see step_kernel)
-      e = launch_chained(ts & 1 ? odd : even, dim3(grid), dim3(WIDE_THREADS), b->side, wid,
-                         (const WideSegment *)w.segs, w.nsegs, (const int *)w.running, b->acc, save, test,
+      e = launch_chained(ts & 1 ? odd : even, dim3(grid), dim3(WIDE_THREADS), sw, wid, (const WideSegment *)w.segs,
+                         w.nsegs, (const int *)w.running, b->acc, save, test,
                          grid - b->sms * wide_min_blocks<true>());
       since++;
       if (e == cudaSuccess && (test || last)) {
-        e = launch_chained(batch_wide_finish_kernel, dim3((w.nwide + 127) / 128), dim3(128), b->side, wid,
+        e = launch_chained(batch_wide_finish_kernel, dim3((w.nwide + 127) / 128), dim3(128), sw, wid,
                            (const int *)w.wide, w.nwide, w.running, b->acc, since, test, ts + 1 >= wid.max_steps, last);
         since = 0;
       }
     }
   }
-  if (e == cudaSuccess) e = cudaEventRecord(b->join, b->side);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b->join, 0);
-  if (e == cudaSuccess) e = cudaEventRecord(b->join_blocks, b->blocks);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b->join_blocks, 0);
+  for (int k = 0; k < forks; k++) {
+    cudaError_t ej = cudaEventRecord(b->join[k], b->side[k]);
+    if (ej == cudaSuccess) ej = cudaStreamWaitEvent(st, b->join[k], 0);
+    if (e == cudaSuccess) e = ej;
+  }
   return e;
 }
 
@@ -798,11 +805,13 @@ extern "C" lbmc_status lbmc_batch_init(const lbmc_batch_config *cfg, int ndomain
   // DMA lands, and the non-blocking streams below do not wait for it.
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
+  // A stream for each class of domains beside the first (~50 us each).
+  const int classes = (b->n_resident > 0) + (b->n_block > 0) + (b->n_resident + b->n_block < ndomains);
+  for (int k = 0; k < classes - 1; k++) {
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming);
+  }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->blocks, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join_blocks, cudaEventDisableTiming);
   if (e == cudaSuccess) {
     switch (cfg->storage) {
       case LBMC_F16: e = configure_batch<__half>(b); break;
@@ -897,49 +906,72 @@ extern "C" lbmc_status lbmc_batch_run(lbmc_batch *b, long long max_steps, double
     b->steps = bs;
   }
 
-  // One launch (queue reset + the kernels of K steps) is captured in a graph
-  // and replayed.  The graph fixes the parity of each step and the steps that
-  // test, so it serves where K is even and a multiple of the check interval
-  // (the tuned ones are), after the first test; other launches, and the last
-  // one before the step cap, are enqueued as they are.  Once a quarter of the
-  // listed wide domains have stopped, their segments are rebuilt and the graph
-  // re-captured, so launches no longer visit them; the same when the
-  // block-stepped domains join the wide path.
-  auto replayable = [&]() {
-    return b->steps % 2 == 0 && b->steps % check_every == 0 && b->t >= check_every && b->t % 2 == 0 &&
-           b->t % check_every == 0 && b->t + b->steps < max_steps;
+  // A launch group (queue reset + the kernels of K steps) is captured in a
+  // graph and replayed.  With wide domains listed, a graph fixes the parity of
+  // its first step and the steps that test, so there is one for each of the
+  // two that comes up: one alone where K is even and a multiple of the check
+  // interval (the tuned ones are) or nothing is wide, else up to GRAPHS, each
+  // captured when its pattern has come up twice before.  The first group and
+  // the last one before the step cap are enqueued as they are.  Once a quarter
+  // of the listed wide domains have stopped, their segments are rebuilt and
+  // the graphs re-captured, so launches no longer visit them; the same when
+  // the block-stepped domains join the wide path.  (us a launch group of one
+  // 16x16 domain, K = 1: 29 enqueued in three branches, 25 replayed in one.)
+  struct Replay {
+    int seen = 0;
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
   };
-  auto capture = [&](cudaGraph_t &graph, cudaGraphExec_t &exec) -> cudaError_t {
+  constexpr int GRAPHS = 32;
+  std::map<long long, Replay> replays;
+  int captured = 0;
+  auto capture = [&](Replay &r) -> cudaError_t {
     cudaError_t ec = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (ec != cudaSuccess) return ec;
     cudaError_t e2 = enqueue_any(b->steps, b->threads);
-    ec = cudaStreamEndCapture(b->stream, &graph);
+    ec = cudaStreamEndCapture(b->stream, &r.graph);
     if (e2 != cudaSuccess) ec = e2;
-    if (ec == cudaSuccess) ec = cudaGraphInstantiate(&exec, graph, 0);
+    if (ec == cudaSuccess) ec = cudaGraphInstantiate(&r.exec, r.graph, 0);
+    captured++;
     return ec;
   };
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  auto drop_graph = [&]() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+  // The next group's graph; null where it is enqueued as it is.
+  auto replay = [&](cudaGraphExec_t &exec) -> cudaError_t {
     exec = nullptr;
-    graph = nullptr;
+    if (b->t + b->steps >= max_steps || (w.nwide > 0 && b->t == 0)) return cudaSuccess;
+    long long pattern = 0;
+    if (w.nwide > 0) {
+      const long long to_test = (check_every - b->t % check_every) % check_every;
+      pattern = 2 * std::min<long long>(to_test, b->steps) + b->t % 2;
+    }
+    Replay &r = replays[pattern];
+    const bool only_one = w.nwide == 0 || (b->steps % 2 == 0 && b->steps % check_every == 0);
+    if (!r.exec && (only_one || r.seen++ >= 2) && captured < GRAPHS) {
+      const cudaError_t ec = capture(r);
+      if (ec != cudaSuccess) return ec;
+    }
+    exec = r.exec;
+    return cudaSuccess;
+  };
+  auto drop_graphs = [&]() {
+    for (auto &r : replays) {
+      if (r.second.exec) cudaGraphExecDestroy(r.second.exec);
+      if (r.second.graph) cudaGraphDestroy(r.second.graph);
+    }
+    replays.clear();
+    captured = 0;
   };
   auto rebuild = [&]() -> cudaError_t {
-    drop_graph();
+    drop_graphs();
     w.release();
     return build_wide(b, all_wide, w);
   };
   int counts[5] = {0, 0, 1, 0, 0};
   const long long launches_max = max_steps / std::max(1, b->steps) + 2;
   for (long long l = 0; e == cudaSuccess && counts[2] > 0 && l < launches_max; l++) {
-    if (replayable()) {
-      if (!exec) e = capture(graph, exec);
-      if (e == cudaSuccess) e = cudaGraphLaunch(exec, b->stream);
-    } else {
-      e = enqueue_any(b->steps, b->threads);
-    }
+    cudaGraphExec_t exec = nullptr;
+    e = replay(exec);
+    if (e == cudaSuccess) e = exec ? cudaGraphLaunch(exec, b->stream) : enqueue_any(b->steps, b->threads);
     b->t = std::min(max_steps, b->t + b->steps);
     if (e == cudaSuccess) e = cudaMemcpyAsync(counts, b->counters, sizeof(counts), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -951,7 +983,7 @@ extern "C" lbmc_status lbmc_batch_run(lbmc_batch *b, long long max_steps, double
       e = rebuild();
     }
   }
-  drop_graph();
+  drop_graphs();
   w.release();
   if (e != cudaSuccess) return berr(LBMC_ERR_CUDA, std::string("lbmc_batch_run: ") + cudaGetErrorString(e));
   if (results) {
@@ -1075,11 +1107,10 @@ extern "C" lbmc_status lbmc_batch_destroy(lbmc_batch *b) {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (b->stream) cudaStreamDestroy(b->stream);
-  if (b->side) cudaStreamDestroy(b->side);
-  if (b->fork) cudaEventDestroy(b->fork);
-  if (b->join) cudaEventDestroy(b->join);
-  if (b->blocks) cudaStreamDestroy(b->blocks);
-  if (b->join_blocks) cudaEventDestroy(b->join_blocks);
+  for (cudaStream_t side : b->side)
+    if (side) cudaStreamDestroy(side);
+  for (cudaEvent_t ev : {b->fork, b->join[0], b->join[1]})
+    if (ev) cudaEventDestroy(ev);
   delete b;
   return LBMC_OK;
 }
