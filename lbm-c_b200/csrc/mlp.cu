@@ -128,6 +128,9 @@ __global__ void __launch_bounds__(GRAD_BLOCK, 1)
   for (int i = 0; i < MLP_H; i++) gw2[i] = 0.f;
   const float inv_b = 1.0f / (float)B;
   for (; first < B; first += stride) {
+    // Samples past the batch count nothing, also where the network overflows
+    // on their zero inputs.
+    auto live = [&](int s) { return first + s < B; };
     __syncwarp();
     // Layer 1: a = W1 x + b1; h1 = silu(a), p1 = silu'(a).
     float p1[GRAD_GROUP], h[GRAD_GROUP];
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(GRAD_BLOCK, 1)
 #pragma unroll
       for (int q = 0; q < MLP_IN; q++) a += w1[q] * x_of[warp][s][q];
       const float sg = sigmoidf_(a);
-      h[s] = a * sg;
+      h[s] = live(s) ? a * sg : 0.f;
       p1[s] = sg + h[s] * (1.0f - sg);
     }
     h1_of[warp][lane] = make_float4(h[0], h[1], h[2], h[3]);
@@ -154,17 +157,16 @@ __global__ void __launch_bounds__(GRAD_BLOCK, 1)
 #pragma unroll
     for (int s = 0; s < GRAD_GROUP; s++) {
       const float sg = sigmoidf_(a2[s]);
-      const float h2 = a2[s] * sg;
+      const float h2 = live(s) ? a2[s] * sg : 0.f;
       float y = w3 * h2;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) y += __shfl_xor_sync(0xffffffffu, y, off);
-      // samples past the batch count nothing
-      const float r = first + s < B ? y + b3 - x_of[warp][s][MLP_IN] : 0.f;
+      const float r = live(s) ? y + b3 - x_of[warp][s][MLP_IN] : 0.f;
       const float dy = 2.0f * r * inv_b;
       loss += r * r * inv_b;
       gb3 += dy;
       gw3 += dy * h2;
-      d2[s] = dy * w3 * (sg + h2 * (1.0f - sg));
+      d2[s] = live(s) ? dy * w3 * (sg + h2 * (1.0f - sg)) : 0.f;
       gb2 += d2[s];
     }
     d2_of[warp][lane] = make_float4(d2[0], d2[1], d2[2], d2[3]);
