@@ -1,9 +1,8 @@
 // Batched persistent step for many independent small D2Q9 domains
 // (lbmc_batch_*).  No counterpart in the reference, which runs one domain per
 // process; each domain here is stepped exactly as lbmc_iterate steps a single
-// domain (the shift layout with FP32 storage and the AA pattern of
-// LBMC_STREAM_AA with 2-byte storage, the same collide_fluid), so parity is
-// inherited.
+// domain (the AA pattern of LBMC_STREAM_AA, the same collide_fluid), so parity
+// is inherited.
 //
 // Execution model.  Domains whose populations fit in a block's shared
 // memory are stepped by one persistent kernel: blocks take whole domains

@@ -5,8 +5,10 @@
 // LBM-C/model_builder.cu:63-248): it validates the configuration, packs the
 // per-node inputs (Porosity, MacroBC, MicroBC) into one class byte per node
 // plus a class table, uploads the fields and sets the initial populations.
-// lbmc_iterate replaces iterate(t) (LBM-C/index.cu:284-313) and enqueues one
-// fused step kernel per time step on the handle's stream; lbmc_fetch replaces
+// lbmc_iterate replaces iterate(t) (LBM-C/index.cu:284-313) and enqueues
+// fused step kernels on the handle's stream: one per time step, several slabs
+// per step in a sweep (sweep.h), or one for many steps of a small 2-D domain;
+// lbmc_fetch replaces
 // the device-to-host copies of output_macros / screen_mess /
 // compute_residual (LBM-C/index.cu:196-216, 387-439).
 #include <cuda_runtime.h>

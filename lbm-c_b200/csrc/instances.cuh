@@ -12,6 +12,8 @@ namespace lbmc {
 // per SM.
 constexpr long long PIPE_STAGE_BUDGET = 32 * 1024;
 
+// The chip this is written for: a slice of it (fewer SMs) only shifts where
+// the last wave begins.
 constexpr int B200_SMS = 148;
 // Dynamic shared memory of a resident block at most: two buffers of 1024
 // D2Q9 nodes in FP64.
@@ -89,8 +91,8 @@ struct Launchers {
   // Whether a block of the direct kernel may take two planes one after the
   // other: that halves the blocks, whose start-up (dispatch, parameters) costs
   // the steps that HBM does not hold back.  Tiled AA, us a step with one and
-  // two planes: BF16 Smagorinsky 256^3 236 and 227, FP16 with stochastic rounding
-  // 250 and 245, D2Q9 FP32 4096x2048 102 and 89; FP32 D3Q15 256^3 254 and 258.
+  // two planes: BF16 Smagorinsky 256^3 236 and 230, FP16 with stochastic rounding
+  // 250 and 247, D2Q9 FP32 4096x2048 102 and 89; FP32 D3Q15 256^3 254 and 258.
   template <int COL>
   static constexpr bool two_planes() {
     return (sizeof(S) == 2 || L::DIM == 2) && !learned_closure(COL);
@@ -105,7 +107,7 @@ struct Launchers {
     return swept || (L::DIM == 2 && (long long)g.x * g.y * g.z >= 16 * wave(d)) ? 2 : 1;
   }
 
-  // One block row per (y, z); blocks of up to STEP_BLOCK threads along x.
+  // One block row per (y, z); blocks of up to DIRECT_BLOCK threads along x.
   static dim3 block_dim(const DeviceState &d) {
     int bx = (d.L[0] + 31) / 32 * 32;
     return dim3(bx < DIRECT_BLOCK ? bx : DIRECT_BLOCK, 1, 1);

@@ -313,7 +313,6 @@ constexpr int DIAG_VALUES = 5;  // mass, momentum x/y/z, kinetic energy
 constexpr int FINALIZE_BLOCKS = 256;
 constexpr int FINALIZE_THREADS = 640;  // 20 warps, a multiple of DIAG_VALUES
 static_assert(FINALIZE_THREADS % DIAG_VALUES == 0, "a thread must meet one diagnostic value");
-constexpr int STEP_BLOCK = 256;  // largest block of any step kernel
 // Direct-load kernel: 64-thread blocks and a register cap that keeps 20 of
 // them (40 warps) resident per SM; measured on B200 to beat 128/256-thread
 // blocks and uncapped registers on the porous D3Q15 workload.
@@ -1372,62 +1371,64 @@ __global__ void __launch_bounds__(DIRECT_BLOCK, (direct_min_blocks<S, COL>()))
       wait_for_predecessor();
 #pragma unroll 1
       for (int part = 0; part < PLANES; part++) {
-      if (part > 0) {  // the block's next plane, unless the launch ends before it
-        int &plane = L::DIM == 3 ? cz : cy;
-        if (plane + 1 == a.end_plane) break;
-        plane = wrap_add(plane, 1, a.L[L::DIM - 1]);
-      }
-      const C inv_scale = a.inv_scale, scale = a.scale;
-      Sites st;
-      TiledSites ts;
-      init_sites(st, ts);
-      int n;
-      if constexpr (FLAT) {
-        const unsigned m = (unsigned)a.first_node + (unsigned)x;
-        n = (int)(m >= (unsigned)a.n ? m - (unsigned)a.n : m);
-      } else {
-        n = x + a.L[0] * (cy + a.L[1] * cz);
-      }
-      S *f = reinterpret_cast<S *>(a.f);
-      Node<L, C> nd;
-      unroll<Q>([&](auto ic) { nd.g[decltype(ic)::value] = load_dev(read_at(f, st, ts, n, ic), inv_scale); });
-      const int cls = a.cls[n];
-      C out[Q];
-      if (cls == CLASS_SOLID) {
-        collide_solid(nd, out);
-      } else {
-        moments(nd);
-        collide_fluid<L, C, COL, FORCE, BLEND>(nd, a, n, cls ? a.table[cls] : 0u, out);
-      }
-      // The store addresses equal the load addresses.  Recomputing them
-      // from the three 32-bit x offsets is cheaper than keeping Q 64-bit
-      // pointers live across the collision, which spills at this kernel's
-      // register cap: 88-116 bytes in the tiled odd step (13% slower with
-      // FP16/BF16 storage), 20-48 bytes in the shift and plain odd maps.
-      // The 2-byte storages, bound by instruction issue, keep the spill in
-      // the plain maps (the recomputation measured slower there).  The
-      // empty asm hides the equality from the compiler.
-      constexpr bool recompute = STREAM == STREAM_AAT_ODD ||
-                                 ((STREAM == STREAM_AA_ODD || STREAM == STREAM_SHIFT) && sizeof(S) >= 4);
-      auto store_all = [&](const Sites &sw, const TiledSites &tw) {
-        if constexpr (stochastic_storage<S>())
-          store_node_sr<Q, true>(out, scale, (unsigned)n ^ a.sr_seed,
-                                 [&](auto ic) { return write_at(f, sw, tw, n, ic); });
-        else if constexpr (std::is_same<S, __half>::value)
-          store_node_f16<Q>(out, scale, [&](auto ic) { return write_at(f, sw, tw, n, ic); });
-        else
-          unroll<Q>([&](auto ic) { store_dev(write_at(f, sw, tw, n, ic), out[decltype(ic)::value], scale, l2_policy(a.keep)); });
-      };
-      if constexpr (recompute) {
-        TiledSites tw = ts;
-        Sites sw = st;
-        if constexpr (STREAM == STREAM_AAT_ODD) asm("" : "+r"(tw.x[0]), "+r"(tw.x[1]), "+r"(tw.x[2]));
-        else asm("" : "+r"(sw.x[0]), "+r"(sw.x[1]), "+r"(sw.x[2]));
-        store_all(sw, tw);
-      } else {
-        store_all(st, ts);
-      }
-      store_and_reduce(nd, a, n, dv, nonfinite, DIAG);
+        if (part > 0) {  // the block's next plane, unless the launch ends before it
+          int &plane = L::DIM == 3 ? cz : cy;
+          if (plane + 1 == a.end_plane) break;
+          plane = wrap_add(plane, 1, a.L[L::DIM - 1]);
+        }
+        const C inv_scale = a.inv_scale, scale = a.scale;
+        Sites st;
+        TiledSites ts;
+        init_sites(st, ts);
+        int n;
+        if constexpr (FLAT) {
+          const unsigned m = (unsigned)a.first_node + (unsigned)x;
+          n = (int)(m >= (unsigned)a.n ? m - (unsigned)a.n : m);
+        } else {
+          n = x + a.L[0] * (cy + a.L[1] * cz);
+        }
+        S *f = reinterpret_cast<S *>(a.f);
+        Node<L, C> nd;
+        unroll<Q>([&](auto ic) { nd.g[decltype(ic)::value] = load_dev(read_at(f, st, ts, n, ic), inv_scale); });
+        const int cls = a.cls[n];
+        C out[Q];
+        if (cls == CLASS_SOLID) {
+          collide_solid(nd, out);
+        } else {
+          moments(nd);
+          collide_fluid<L, C, COL, FORCE, BLEND>(nd, a, n, cls ? a.table[cls] : 0u, out);
+        }
+        // The store addresses equal the load addresses.  Recomputing them
+        // from the three 32-bit x offsets is cheaper than keeping Q 64-bit
+        // pointers live across the collision, which spills at this kernel's
+        // register cap: 88-116 bytes in the tiled odd step (13% slower with
+        // FP16/BF16 storage), 20-48 bytes in the shift and plain odd maps.
+        // The 2-byte storages, bound by instruction issue, keep the spill in
+        // the plain maps (the recomputation measured slower there).  The
+        // empty asm hides the equality from the compiler.
+        constexpr bool recompute = STREAM == STREAM_AAT_ODD ||
+                                   ((STREAM == STREAM_AA_ODD || STREAM == STREAM_SHIFT) && sizeof(S) >= 4);
+        auto store_all = [&](const Sites &sw, const TiledSites &tw) {
+          if constexpr (stochastic_storage<S>())
+            store_node_sr<Q, true>(out, scale, (unsigned)n ^ a.sr_seed,
+                                   [&](auto ic) { return write_at(f, sw, tw, n, ic); });
+          else if constexpr (std::is_same<S, __half>::value)
+            store_node_f16<Q>(out, scale, [&](auto ic) { return write_at(f, sw, tw, n, ic); });
+          else
+            unroll<Q>([&](auto ic) {
+              store_dev(write_at(f, sw, tw, n, ic), out[decltype(ic)::value], scale, l2_policy(a.keep));
+            });
+        };
+        if constexpr (recompute) {
+          TiledSites tw = ts;
+          Sites sw = st;
+          if constexpr (STREAM == STREAM_AAT_ODD) asm("" : "+r"(tw.x[0]), "+r"(tw.x[1]), "+r"(tw.x[2]));
+          else asm("" : "+r"(sw.x[0]), "+r"(sw.x[1]), "+r"(sw.x[2]));
+          store_all(sw, tw);
+        } else {
+          store_all(st, ts);
+        }
+        store_and_reduce(nd, a, n, dv, nonfinite, DIAG);
       }
     }
   } else {
@@ -1501,7 +1502,11 @@ __device__ __forceinline__ unsigned smem_addr(const void *p) {
 // node's own slots of the other buffer, and ends in one cluster barrier.  The
 // state comes from and goes back to the handle's layout, and every population
 // is rounded to its storage type at every step, so the results are those of
-// single steps.  128x64: 100 steps with their synchronisation 409 -> 116 us
+// single steps, bit for bit (in FP64 as far as the compiler fuses the same
+// multiplies and adds in both kernels, which it does in every variant).  FP64
+// spills up to 184 bytes a thread at the cap of 64 registers where a block
+// holds more than 512 nodes; 128x128 still takes 1.8 us a step (Smagorinsky
+// 2.4) against 4.3 step by step.  128x64: 100 steps with their synchronisation 409 -> 116 us
 // (1.05 us a step).  Bound by instruction issue on the 16 SMs of a cluster (16
 // warps x ~280 instructions over 4 schedulers are 0.6 us) and the barrier.
 constexpr int RESIDENT_MAX_CLUSTER = 16;

@@ -46,7 +46,8 @@ struct SweepPlan {
 // storage elements of elem bytes.  Measured on a B200 (126 MB L2), us per
 // step, step by step -> swept: D3Q15 MRT 256^3 FP32 326 -> 255 (65.7 GLUPS; one
 // read and one write of HBM per step would allow 54), FP16 with stochastic
-// rounding 262 -> 250, Smagorinsky 256^3 BF16 259 -> 236, 160^3 FP64 181 -> 137,
+// rounding 262 -> 247, Smagorinsky 256^3 BF16 259 -> 230 (both with two planes
+// a block; 250 and 236 with one), 160^3 FP64 181 -> 137,
 // 192^3 FP32 140 -> 107, D2Q9 4096x2048 FP32 115 -> 103.
 //   - Slabs of ~30 MB: 16 MB ones (256^3 FP32, 4 planes) lose to the drain
 //     between launches, 47 MB ones (12 planes: 294) to evictions.
